@@ -44,6 +44,7 @@
 #else
 #define PTM_CALL static __device__ __forceinline__
 #endif
+#define PTM_COLD static __device__ __noinline__ /* rare paths */
 #define PTM_FMA(a, b, c) __fmaf_rn((a), (b), (c))
 PTM_FN uint32_t ptm_bits(float f) { return __float_as_uint(f); }
 PTM_FN float ptm_from_bits(uint32_t u) { return __uint_as_float(u); }
@@ -52,6 +53,7 @@ PTM_FN float ptm_from_bits(uint32_t u) { return __uint_as_float(u); }
 #include <string.h>
 #define PTM_FN static inline
 #define PTM_CALL static inline
+#define PTM_COLD static inline
 #define PTM_FMA(a, b, c) fmaf((a), (b), (c))
 PTM_FN uint32_t ptm_bits(float f) {
     uint32_t u;
@@ -119,42 +121,58 @@ typedef struct ptm_sc {
     float s, c;
 } ptm_sc;
 
-/* sin and cos of x together. */
-PTM_FN ptm_sc ptm_sincos_inline(float x) {
+/* The sum x + PTM_RINT_MAGIC (1.5 * 2^23) rounds x to the nearest integer,
+ * ties to even, for |x| < 2^22, and holds that integer in its low mantissa
+ * bits: rintf and the conversion to int in one addition.  On GB300 the two
+ * conversion instructions it stands for occupy their unit for 8 cycles per
+ * warp each (measured; an addition 1), which bound the functions below. */
+#define PTM_RINT_MAGIC 12582912.0f
+#define PTM_RINT_MAGIC_BITS 0x4b400000u
+
+/* sin and cos from the reduced argument r and the quadrant q (mod 4). */
+PTM_FN ptm_sc ptm_sincos_quadrant(float r, uint32_t q) {
+    const float z = r * r;
+    const float p = PTM_FMA(PTM_FMA(PTM_FMA(PTM_S3, z, PTM_S2), z, PTM_S1), z, PTM_S0);
+    const float sr = PTM_FMA(r * z, p, r);
+    const float qc = PTM_FMA(PTM_FMA(PTM_FMA(PTM_C3, z, PTM_C2), z, PTM_C1), z, PTM_C0);
+    const float cr = PTM_FMA(z * z, qc, PTM_FMA(-0.5f, z, 1.0f));
+    const float s = (q & 1u) ? cr : sr, c = (q & 1u) ? sr : cr;
     ptm_sc out;
+    out.s = ptm_from_bits(ptm_bits(s) ^ ((q << 30) & 0x80000000u));         /* negative in quadrants 2, 3 */
+    out.c = ptm_from_bits(ptm_bits(c) ^ (((q + 1u) << 30) & 0x80000000u));  /* negative in quadrants 1, 2 */
+    return out;
+}
+
+PTM_FN float ptm_sincos_reduce(float x, float k) {
+    float r = PTM_FMA(-k, PTM_PIO2_1, x);
+    r = PTM_FMA(-k, PTM_PIO2_2, r);
+    return PTM_FMA(-k, PTM_PIO2_3, r);
+}
+
+/* |x| 2/pi >= 2^22, inf or NaN: the same reduction with a general rounding. */
+PTM_COLD ptm_sc ptm_sincos_large(float x) {
     if (!(x - x == 0.0f)) { /* inf or NaN */
+        ptm_sc out;
         out.s = PTM_NAN;
         out.c = PTM_NAN;
         return out;
     }
     const float k = rintf(x * PTM_2_OVER_PI);
-    float r = PTM_FMA(-k, PTM_PIO2_1, x);
-    r = PTM_FMA(-k, PTM_PIO2_2, r);
-    r = PTM_FMA(-k, PTM_PIO2_3, r);
     /* k mod 4, exact for every finite k */
     const int q = (int)(k - 4.0f * floorf(k * 0.25f));
-    const float z = r * r;
-    float p = PTM_FMA(PTM_FMA(PTM_FMA(PTM_S3, z, PTM_S2), z, PTM_S1), z, PTM_S0);
-    const float sr = PTM_FMA(r * z, p, r);
-    float qc = PTM_FMA(PTM_FMA(PTM_FMA(PTM_C3, z, PTM_C2), z, PTM_C1), z, PTM_C0);
-    const float cr = PTM_FMA(z * z, qc, PTM_FMA(-0.5f, z, 1.0f));
-    float s, c;
-    if (q == 0) {
-        s = sr;
-        c = cr;
-    } else if (q == 1) {
-        s = cr;
-        c = -sr;
-    } else if (q == 2) {
-        s = -sr;
-        c = -cr;
-    } else {
-        s = -cr;
-        c = sr;
-    }
-    out.s = s;
-    out.c = c;
-    return out;
+    return ptm_sincos_quadrant(ptm_sincos_reduce(x, k), (uint32_t)q);
+}
+
+/* sin and cos of x together, for |x| 2/pi < 2^22. */
+PTM_FN ptm_sc ptm_sincos_small(float x) {
+    const float kb = x * PTM_2_OVER_PI + PTM_RINT_MAGIC;
+    return ptm_sincos_quadrant(ptm_sincos_reduce(x, kb - PTM_RINT_MAGIC), ptm_bits(kb));
+}
+
+/* sin and cos of x together. */
+PTM_FN ptm_sc ptm_sincos_inline(float x) {
+    if (!(fabsf(x * PTM_2_OVER_PI) < 4194304.0f)) return ptm_sincos_large(x);
+    return ptm_sincos_small(x);
 }
 
 PTM_CALL ptm_sc ptm_sincos_v(float x) { return ptm_sincos_inline(x); }
@@ -181,6 +199,7 @@ PTM_FN float ptm_cosf(float x) {
 
 /* y * 2^k for integral k in [-300, 300], exact unless the result is subnormal. */
 PTM_FN float ptm_scale2(float y, int k) {
+    if ((uint32_t)(k + 126) <= 253u) return y * ptm_from_bits((uint32_t)(k + 127) << 23);
     if (k > 127) {
         y *= ptm_from_bits(0x7f000000u); /* 2^127 */
         k -= 127;
@@ -197,13 +216,14 @@ PTM_CALL float ptm_expf(float x) {
     if (x != x) return x;
     if (x > 88.72283936f) return PTM_INF;
     if (x < -103.9720840f) return 0.0f;
-    const float k = rintf(x * PTM_LOG2E);
+    const float kb = x * PTM_LOG2E + PTM_RINT_MAGIC;
+    const float k = kb - PTM_RINT_MAGIC;
     float r = PTM_FMA(-k, PTM_LN2_1, x);
     r = PTM_FMA(-k, PTM_LN2_2, r);
     const float p =
         PTM_FMA(PTM_FMA(PTM_FMA(PTM_FMA(PTM_FMA(PTM_E5, r, PTM_E4), r, PTM_E3), r, PTM_E2), r, PTM_E1), r, PTM_E0);
     const float em1 = PTM_FMA(r * r, p, r); /* e^r - 1 */
-    return ptm_scale2(1.0f + em1, (int)k);
+    return ptm_scale2(1.0f + em1, (int)(ptm_bits(kb) - PTM_RINT_MAGIC_BITS));
 }
 
 /* log(1+f) for f = m - 1, m in [sqrt(1/2), sqrt(2)]. */
@@ -242,7 +262,7 @@ PTM_FN float ptm_logf_inline(float x) {
     int e;
     const float m = ptm_frexp_sqrt2(x, &e);
     const float l1p = ptm_log1p_reduced(m - 1.0f);
-    const float ef = (float)e;
+    const float ef = ptm_from_bits(PTM_RINT_MAGIC_BITS + (uint32_t)e) - PTM_RINT_MAGIC; /* (float)e */
     return PTM_FMA(ef, PTM_LN2_1, PTM_FMA(ef, PTM_LN2_2, l1p));
 }
 
@@ -385,13 +405,13 @@ PTM_CALL float ptm_exp2f(float x) {
     if (x != x) return x;
     if (x > 128.0f) return PTM_INF;
     if (x < -150.0f) return 0.0f;
-    const float k = rintf(x);
-    const float f = x - k;
+    const float kb = x + PTM_RINT_MAGIC;
+    const float f = x - (kb - PTM_RINT_MAGIC);
     const float r = PTM_FMA(f, PTM_LN2_1, f * PTM_LN2_2);
     const float p =
         PTM_FMA(PTM_FMA(PTM_FMA(PTM_FMA(PTM_FMA(PTM_E5, r, PTM_E4), r, PTM_E3), r, PTM_E2), r, PTM_E1), r, PTM_E0);
     const float em1 = PTM_FMA(r * r, p, r);
-    return ptm_scale2(1.0f + em1, (int)k);
+    return ptm_scale2(1.0f + em1, (int)(ptm_bits(kb) - PTM_RINT_MAGIC_BITS));
 }
 
 /* log2(x) = log(x) * log2(e). */

@@ -1,0 +1,110 @@
+"""Exact shortcuts of the float path: forms that replace slower ones must give
+the same bits, checked here on the CPU against the plain forms."""
+import os
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+MATHF_C = r"""
+#include "pt_mathf.h"
+/* the functions with rintf and float-to-int conversions in place of the magic addition */
+static float scale2(float y, int k) {
+    if (k > 127) { y *= ptm_from_bits(0x7f000000u); k -= 127; if (k > 127) k = 127; }
+    else if (k < -126) { y *= ptm_from_bits(0x00800000u); k += 126; if (k < -126) k = -126; }
+    return y * ptm_from_bits((uint32_t)(k + 127) << 23);
+}
+static float epoly(float r) {
+    const float p = PTM_FMA(PTM_FMA(PTM_FMA(PTM_FMA(PTM_FMA(PTM_E5, r, PTM_E4), r, PTM_E3), r, PTM_E2), r, PTM_E1), r, PTM_E0);
+    return 1.0f + PTM_FMA(r * r, p, r);
+}
+static float exp_plain(float x) {
+    if (x != x) return x;
+    if (x > 88.72283936f) return PTM_INF;
+    if (x < -103.9720840f) return 0.0f;
+    const float k = rintf(x * PTM_LOG2E);
+    float r = PTM_FMA(-k, PTM_LN2_1, x);
+    r = PTM_FMA(-k, PTM_LN2_2, r);
+    return scale2(epoly(r), (int)k);
+}
+static float exp2_plain(float x) {
+    if (x != x) return x;
+    if (x > 128.0f) return PTM_INF;
+    if (x < -150.0f) return 0.0f;
+    const float k = rintf(x), f = x - k;
+    return scale2(epoly(PTM_FMA(f, PTM_LN2_1, f * PTM_LN2_2)), (int)k);
+}
+static float log_plain(float x) {
+    if (x != x) return x;
+    if (x < 0.0f) return PTM_NAN;
+    if (x == 0.0f) return -PTM_INF;
+    if (x == PTM_INF) return x;
+    int e;
+    const float m = ptm_frexp_sqrt2(x, &e), ef = (float)e;
+    return PTM_FMA(ef, PTM_LN2_1, PTM_FMA(ef, PTM_LN2_2, ptm_log1p_reduced(m - 1.0f)));
+}
+static void sincos_plain(float x, float* s, float* c) {
+    if (!(x - x == 0.0f)) { *s = *c = PTM_NAN; return; }
+    const float k = rintf(x * PTM_2_OVER_PI);
+    float r = PTM_FMA(-k, PTM_PIO2_1, x);
+    r = PTM_FMA(-k, PTM_PIO2_2, r);
+    r = PTM_FMA(-k, PTM_PIO2_3, r);
+    const int q = (int)(k - 4.0f * floorf(k * 0.25f));
+    const float z = r * r;
+    const float sr = PTM_FMA(r * z, PTM_FMA(PTM_FMA(PTM_FMA(PTM_S3, z, PTM_S2), z, PTM_S1), z, PTM_S0), r);
+    const float cr = PTM_FMA(z * z, PTM_FMA(PTM_FMA(PTM_FMA(PTM_C3, z, PTM_C2), z, PTM_C1), z, PTM_C0), PTM_FMA(-0.5f, z, 1.0f));
+    *s = q == 0 ? sr : q == 1 ? cr : q == 2 ? -sr : -cr;
+    *c = q == 0 ? cr : q == 1 ? -sr : q == 2 ? -cr : sr;
+}
+long forms_differ(uint32_t first, uint32_t step) {
+    long bad = 0;
+    uint64_t u;
+    for (u = first; u < (1ull << 32); u += step) {
+        const float x = ptm_from_bits((uint32_t)u);
+        float s, c;
+        sincos_plain(x, &s, &c);
+        const ptm_sc v = ptm_sincos_inline(x);
+        bad += ptm_bits(v.s) != ptm_bits(s) || ptm_bits(v.c) != ptm_bits(c);
+        bad += ptm_bits(ptm_expf(x)) != ptm_bits(exp_plain(x));
+        bad += ptm_bits(ptm_exp2f(x)) != ptm_bits(exp2_plain(x));
+        bad += ptm_bits(ptm_logf(x)) != ptm_bits(log_plain(x));
+    }
+    return bad;
+}
+/* c * hi + c * lo against c / divisor for every significand, both signs, in two binades */
+long quotients_differ(float divisor, float hi, float lo) {
+    long bad = 0;
+    uint32_t m;
+    int e, sign;
+    for (m = 0; m < (1u << 23); m++)
+        for (e = 103; e <= 127; e += 24)
+            for (sign = 0; sign < 2; sign++) {
+                const float c = ptm_from_bits(((uint32_t)sign << 31) | ((uint32_t)e << 23) | m);
+                bad += ptm_bits(PTM_FMA(c, hi, c * lo)) != ptm_bits(c / divisor);
+            }
+    return bad;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def forms(tmp_path_factory):
+    import ctypes
+
+    d = tmp_path_factory.mktemp("forms")
+    src, out = d / "forms.c", d / "forms.so"
+    src.write_text(MATHF_C)
+    subprocess.run([os.environ.get("CC", "gcc"), "-O2", "-std=c11", "-ffp-contract=off", "-fPIC", "-shared",
+                    "-I" + os.path.join(ROOT, "include"), "-o", str(out), str(src), "-lm"], check=True)
+    lib = ctypes.CDLL(str(out))
+    lib.forms_differ.restype = lib.quotients_differ.restype = ctypes.c_long
+    lib.forms_differ.argtypes = [ctypes.c_uint32, ctypes.c_uint32]
+    lib.quotients_differ.argtypes = [ctypes.c_float] * 3
+    return lib
+
+
+@pytest.mark.parametrize("first", [0, 1, 1234])
+def test_mathf_without_conversions_is_the_plain_form(forms, first):
+    """Every 4099th float (NaNs, infinities, subnormals and both zeros among them)."""
+    assert forms.forms_differ(first, 4099) == 0
