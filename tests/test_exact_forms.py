@@ -1,6 +1,7 @@
 """Exact shortcuts of the float path: forms that replace slower ones must give
 the same bits, checked here on the CPU against the plain forms."""
 import os
+import re
 import subprocess
 
 import pytest
@@ -108,3 +109,14 @@ def forms(tmp_path_factory):
 def test_mathf_without_conversions_is_the_plain_form(forms, first):
     """Every 4099th float (NaNs, infinities, subnormals and both zeros among them)."""
     assert forms.forms_differ(first, 4099) == 0
+
+
+def test_menger_level_division_is_the_quotient(forms):
+    """c / 3^N by its two-part reciprocal, with the constants of sdf_menger."""
+    with open(os.path.join(ROOT, "pathtracer_gb300", "csrc", "kernel", "pt_geometry.cuh")) as f:
+        text = f.read()
+    hi, lo = ([float(x.strip().rstrip("f")) for x in re.search(name + r"\[5\] = \{([^}]*)\}", text).group(1).split(", ")]
+              for name in ("kInvHi", "kInvLo"))
+    for n in range(5):
+        assert forms.quotients_differ(3.0 ** (n + 1), hi[n], lo[n]) == 0
+    assert forms.quotients_differ(9.0, hi[1], 0.0) != 0  # the low part is needed
