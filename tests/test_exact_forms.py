@@ -115,7 +115,7 @@ def test_menger_level_division_is_the_quotient(forms):
     """c / 3^N by its two-part reciprocal, with the constants of sdf_menger."""
     with open(os.path.join(ROOT, "pathtracer_gb300", "csrc", "kernel", "pt_geometry.cuh")) as f:
         text = f.read()
-    hi, lo = ([float(x.strip().rstrip("f")) for x in re.search(name + r"\[5\] = \{([^}]*)\}", text).group(1).split(", ")]
+    hi, lo = ([float(x.strip().rstrip("f")) for x in re.search(name + r"\[5\] = \{([^}]*)\}", text).group(1).split(",")]
               for name in ("kInvHi", "kInvLo"))
     for n in range(5):
         assert forms.quotients_differ(3.0 ** (n + 1), hi[n], lo[n]) == 0
