@@ -172,6 +172,7 @@ PT_DI float3 normal_probes(unsigned pending, const KScene* Sp, float3 p, uint32_
         const uint64_t sp = reinterpret_cast<uint64_t>(Sp);
         const uint32_t lo = __shfl_sync(0xffffffffu, (uint32_t)sp, src);
         const uint32_t hi = __shfl_sync(0xffffffffu, (uint32_t)(sp >> 32), src);
+        const uint32_t walk = __reduce_or_sync(0xffffffffu, probe ? s1 : 0u);
         float val = 0.0f;
         if (probe) {
             const KScene& S = *reinterpret_cast<const KScene*>((uint64_t)lo | ((uint64_t)hi << 32));
@@ -179,7 +180,7 @@ PT_DI float3 normal_probes(unsigned pending, const KScene* Sp, float3 p, uint32_
             const float mx = (j == 1) ? e : 0.0f, my = (j == 3) ? e : 0.0f, mz = (j == 5) ? e : 0.0f;
             const float3 q = (j & 1) ? f3(px - mx, py - my, pz - mz) : f3(px + ex, py + ey, pz + ez);
             int esel = -1;
-            val = scene_sdf_sel(S, q, s1, esel);
+            val = scene_sdf_sel(S, q, s1, walk, esel);
         }
         // Ray lane L collects the probes of its rank among `take`.
         const int base = 6 * __popc(take & ((1u << lane) - 1u));
@@ -360,7 +361,12 @@ PT_DI void march_rays(const WfArgs& A) {
             }
             float val = 0.0f;
             int esel = -1;
-            if (evalLane) val = scene_sdf_sel(*Sp, q, set1, esel);
+#if defined(PT_ONE_SDF)
+            const uint32_t walk = 1u;
+#else
+            const uint32_t walk = __reduce_or_sync(0xffffffffu, evalLane ? set1 : 0u);
+#endif
+            if (evalLane) val = scene_sdf_sel(*Sp, q, set1, walk, esel);
             if (!evalLane) continue;
             if (phase == MP_SIGN) {
                 k = sign_glsl(val);
