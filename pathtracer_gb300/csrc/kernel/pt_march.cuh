@@ -104,6 +104,17 @@ struct PoolView {
     PairField<float4> s9, h0, h1, m0, m1;
 };
 
+// An entry of the shadow queues: the slot (pools have at most 2^28) and what
+// the march kernel found for the shadow ray, so that a marched shadow ray
+// writes nothing else: bit 31 an SDF hit, bits 29-30 the SDF's sign at the
+// ray's origin + 2 (0: not marched).
+constexpr uint32_t kQueueSlotMask = (1u << 28) - 1u;
+constexpr uint32_t kQueueSdfHit = 1u << 31;
+PT_DI uint32_t shadow_entry(uint32_t slot, bool hit, float k) {
+    return slot | (hit ? kQueueSdfHit : 0u) | ((k > 0.0f ? 3u : (k < 0.0f ? 1u : 2u)) << 29);
+}
+PT_DI uint32_t queue_sign(uint32_t entry) { return (entry >> 29) & 3u; }
+
 // The word in m1.z of a suspended march: bit 31 set, the SDF sign k
 // (-1, 0, 1) + 1 in bits 26-27, points in bits 10-25 and the loop
 // iterations in bits 0-9.  A ray fresh from intersection has 0 there.
@@ -420,7 +431,10 @@ PT_DI void march_rays(const WfArgs& A) {
                     if (iter >= (xmarch ? Sp->ext.march_max_steps : 512)) exitLoop = true;
                 }
                 if (exitLoop) {
-                    if (t < hitdist) {
+                    if (shadow_ray) {  // reports only whether an SDF was hit
+                        hit = t < hitdist;
+                        finished = true;
+                    } else if (t < hitdist) {
                         p = fma3s(dir, t, org);
                         phase = WARP_NORMALS ? MP_NORMAL : MP_NORMAL0;
                     } else {
@@ -466,7 +480,7 @@ PT_DI void march_rays(const WfArgs& A) {
                     v.h1[slot] = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
                 }
             }
-        } else if (finished && hit) {
+        } else if (finished && hit && !shadow_ray) {
             const float3 nrm = normalize3(nv);
             const float mat = scene_sdf_material_hit(*Sp, p, set1, hit_sel);
             v.h0[slot] = make_float4(t - 1e-3f, mat, -1.0f, __int_as_float(-2));
@@ -474,7 +488,7 @@ PT_DI void march_rays(const WfArgs& A) {
         }
         stage_push(A, staged[wib][0], nstaged[0], finished && !shadow_ray, slot, A.q_shade[cur], &C.n_shade[cur],
                    lane);
-        stage_push(A, staged[wib][1], nstaged[1], finished && shadow_ray, slot, A.q_shadow[cur], &C.n_shadow[cur],
+        stage_push(A, staged[wib][1], nstaged[1], finished && shadow_ray, shadow_entry(slot, hit, k), A.q_shadow[cur], &C.n_shadow[cur],
                    lane);
         q_push(A, A.q_march[cur ^ 1u], &C.n_march[cur ^ 1u], slot, suspend);
         if (finished || suspend) phase = MP_EMPTY;

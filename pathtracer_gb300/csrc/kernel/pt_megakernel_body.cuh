@@ -53,6 +53,7 @@ __global__ void __launch_bounds__(PT_MK_THREADS) megakernel(const __grid_constan
     int k = 0;
     PathStateT<R> ps;
     bool active = false, shadow = false;
+    OriginSignT<R> sign{R(0), 0u};
     for (;;) {
         if (!active) {
             // Finish sample k-1 (SC:1477-1489, SC:1514-1516) and start sample k.
@@ -73,6 +74,7 @@ __global__ void __launch_bounds__(PT_MK_THREADS) megakernel(const __grid_constan
             start_sample(ps, S, pc, camS, xx, yy, uvx, uvy, k);
             k++;
             shadow = false;
+            sign.set = 0u;
             active = depth > 0;
             continue;
         }
@@ -83,7 +85,8 @@ __global__ void __launch_bounds__(PT_MK_THREADS) megakernel(const __grid_constan
         h.materialID = R(0);
         h.lightID = R(-1);
         int objectID = -1;
-        intersect_all<FEAT>(S, ps.org, shadow ? ps.shDir : ps.dir, h, objectID);
+        intersect_all<FEAT>(S, ps.org, shadow ? ps.shDir : ps.dir, h, objectID, shadow, ps.shObj, sign);
+        if (!shadow) sign.set = 0u;  // shading moves the origin
         const StepResult r =
             shadow ? shade_shadow<TRACE>(ps, S, objectID, depth) : shade_primary<TRACE>(ps, S, h, objectID, depth);
         shadow = (r == STEP_SHADOW);

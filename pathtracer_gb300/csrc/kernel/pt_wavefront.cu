@@ -54,12 +54,13 @@ PT_DI uint32_t bounce_word(const PathState& ps) {
 
 // A shadow-ray result's state: the bounce's next ray (s0, s1), the NEE
 // term and the next throughput made with the shadow ray (s3, s5: see
-// shade_shadow_made), the radiance, wavelengths and RNG/pass words and,
+// shade_shadow_made), the SDF set its march started with (s2.w, in s3's
+// sector), the radiance, wavelengths and RNG/pass words and,
 // traced, the event word.  The light sample's geometry and the BRDF those
 // two came from are not stored, so they are neither read here.
 template <bool TRACE>
-PT_DI void load_for_shadow(const PoolView& v, uint32_t slot, PathState& ps, float4& contrib, uint32_t& flags,
-                           uint32_t& sample, uint32_t& job) {
+PT_DI void load_for_shadow(const PoolView& v, uint32_t slot, PathState& ps, float4& contrib, uint32_t& sign_set,
+                           uint32_t& flags, uint32_t& sample, uint32_t& job) {
     const float4 a = v.s0[slot], b = v.s1[slot];
     ps.org = f3(a.x, a.y, a.z);
     ps.mis = a.w;
@@ -70,6 +71,7 @@ PT_DI void load_for_shadow(const PoolView& v, uint32_t slot, PathState& ps, floa
     ps.nrm = f3(0.0f, 0.0f, 0.0f);
     ps.lightPdf = 0.0f;
     ps.brdf = f4s(0.0f);
+    sign_set = __float_as_uint(v.s2[slot].w);
     contrib = v.s3[slot];
     ps.rr = v.s5[slot];
     ps.radiance = v.s6[slot];
@@ -140,7 +142,12 @@ PT_DI uint64_t jobs_total(const WfArgs& A, uint32_t hi) {
 // primitives, then the SDF bounding boxes.  Writes the hit record and, for a
 // ray that needs sphere tracing, the march start state (the march kernel
 // picks it up like a ray it suspended).  Returns true for such a ray.
-PT_DI bool route_ray(const WfArgs& A, const PoolView& v, const KScene& S, uint32_t slot, float3 org, float3 dir) {
+// `shadow`: a shadow ray towards light object shObj, marched only when an
+// SDF hit can change what it reports.  sign_k: the SDF's sign at the origin
+// as queue_sign gave it for the set sign_set (0: not known); a ray with that
+// set starts past its sign probe.  *set_out: the ray's set (0: no march).
+PT_DI bool route_ray(const WfArgs& A, const PoolView& v, const KScene& S, uint32_t slot, float3 org, float3 dir,
+                     bool shadow, int shObj, uint32_t sign_k, uint32_t sign_set, uint32_t* set_out) {
     Hit h;
     h.hitdist = PT_MAXDIST;
     h.normal = f3(0.0f, 0.0f, 0.0f);
@@ -149,16 +156,19 @@ PT_DI bool route_ray(const WfArgs& A, const PoolView& v, const KScene& S, uint32
     int objectID = -1;
     intersect_analytic(S, org, dir, h, objectID);
     bool march = false;
-    if (S.meta.n[5] > 0) {
+    uint32_t set1 = 0;
+    if (S.meta.n[5] > 0 && !(shadow && !shadow_needs_march(objectID, shObj))) {
         const float3 invdir = f3(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
         float2 tmm = make_float2(PT_MAXDIST, PT_MAXDIST);
-        uint32_t set1 = 0;
         march = search_sdf(S, org, invdir, tmm, set1);
         if (march) {
+            // not suspended, or past the sign probe like a suspended march
+            const uint32_t word = (sign_k != 0u && sign_set == set1) ? march_word((float)((int)sign_k - 2), 0, 0) : 0u;
             v.m0[slot] = make_float4(fmaxf(tmm.x, 1e-3f), 0.0f, kOmegaMax, 0.0f);
-            v.m1[slot] = make_float4(tmm.x, tmm.y, __uint_as_float(0u), __uint_as_float(set1));  // not suspended
+            v.m1[slot] = make_float4(tmm.x, tmm.y, __uint_as_float(word), __uint_as_float(set1));
         }
     }
+    if (set_out) *set_out = march ? set1 : 0u;
     v.h0[slot] = make_float4(h.hitdist, h.materialID, h.lightID, __int_as_float(objectID));
     v.h1[slot] = make_float4(h.normal.x, h.normal.y, h.normal.z, 0.0f);
     return march;
@@ -214,7 +224,7 @@ __global__ void PT_GEN_BOUNDS wf_gen(const __grid_constant__ WfArgs A) {
             ps.shObj = 0;
             ps.ev = 0;
             store_new_sample(v, slot, ps, local, job);
-            march = route_ray(A, v, *J.scene, slot, ps.org, ps.dir);
+            march = route_ray(A, v, *J.scene, slot, ps.org, ps.dir, false, 0, 0u, 0u, nullptr);
         }
         push_routed(A, C, nxt, slot, valid, march, false);
     }
@@ -339,26 +349,30 @@ __global__ void PT_SHADE_BOUNDS wf_shade(const __grid_constant__ WfArgs A) {
         bool valid = i < ns;
         uint32_t slot = 0, job = 0;
         bool again = false, freed = false, march = false;
+        uint32_t entry = 0;
         if (valid) {
-            slot = A.q_shadow[cur][i];
+            entry = A.q_shadow[cur][i];
+            slot = entry & kQueueSlotMask;
             valid = pt_check(A, slot, A.pool_size, PT_CHECK_QUEUE_SLOT) &&
                     pt_check(A, slot_job(v, slot), A.job_cap, PT_CHECK_JOB);
         }
         if (valid) {
             PathState ps;
             float4 contrib;
-            uint32_t flags, sample;
-            load_for_shadow<TRACE>(v, slot, ps, contrib, flags, sample, job);
+            uint32_t flags, sample, sign_set;
+            load_for_shadow<TRACE>(v, slot, ps, contrib, sign_set, flags, sample, job);
             const WfJob& J = A.jobs[job];
-            const int objectID = __float_as_int(v.h0[slot].w);
+            const int objectID = (entry & kQueueSdfHit) ? -2 : __float_as_int(v.h0[slot].w);
             const float4 rr_next = ps.rr;
             const StepResult r = shade_shadow_made<TRACE>(ps, objectID, contrib, rr_next, J.pc.pathLength);
             finish_shade<TRACE>(A, J, ps, r, sample, freed);
             if (!freed) {
                 store_after_shadow(v, slot, ps, sample, job, TRACE);
                 again = true;
-                // the bounce's next primary ray, set up with the primary hit
-                march = route_ray(A, v, *J.scene, slot, ps.org, ps.dir);
+                // the bounce's next primary ray, set up with the primary hit;
+                // it leaves the shadow ray's origin
+                march = route_ray(A, v, *J.scene, slot, ps.org, ps.dir, false, 0, queue_sign(entry), sign_set,
+                                  nullptr);
             }
         }
         push_routed(A, C, nxt, slot, again, march, false);
@@ -392,30 +406,33 @@ __global__ void PT_SHADE_BOUNDS wf_shade(const __grid_constant__ WfArgs A) {
             finish_shade<TRACE>(A, J, ps, r, sample, freed);
             if (!freed) {
                 // the path state.  For a light sample's shadow ray: its
-                // direction (s2, read by the march) and, made now with the
+                // direction and first SDF set (s2) and, made now with the
                 // shadow step's own operations (shade_shadow_made), the NEE
                 // term (s3) and the bounce's next throughput (s5), so the
                 // shadow step reads neither the light sample's geometry nor
                 // the BRDF (s4 is kept only when traced, beside s9).  A next
                 // bounce's primary ray reads none of s2-s4.
+                shadow_next = (r == STEP_SHADOW);
                 v.s0[slot] = make_float4(ps.org.x, ps.org.y, ps.org.z, ps.mis);
                 v.s1[slot] = make_float4(ps.dir.x, ps.dir.y, ps.dir.z, ps.brdfPdf);
-                if (r == STEP_SHADOW) {
-                    v.s2[slot] = make_float4(ps.shDir.x, ps.shDir.y, ps.shDir.z, ps.cosL);
+                if (shadow_next) {
                     v.s3[slot] = shadow_contribution(ps, *J.scene);
                     if (TRACE) v.s4[slot] = ps.brdf;
                 }
-                v.s5[slot] = (r == STEP_SHADOW) ? bounce_throughput(ps) : ps.rr;
+                v.s5[slot] = shadow_next ? bounce_throughput(ps) : ps.rr;
                 v.s6[slot] = ps.radiance;
                 v.s7[slot] = ps.l;  // unchanged: written with s8 so their sector is written whole
-                v.s8[slot] = make_uint4(ps.seed, ((r == STEP_SHADOW) ? kShadowFlag : 0u) | bounce_word(ps), sample,
-                                        job_word(job, ps.shObj));
+                v.s8[slot] =
+                    make_uint4(ps.seed, (shadow_next ? kShadowFlag : 0u) | bounce_word(ps), sample, job_word(job, ps.shObj));
                 // traced: the light picked and the event word
                 if (TRACE) v.s9[slot] = make_float4(ps.shLightID, __uint_as_float(ps.ev), 0.0f, 0.0f);
-                again = true;
                 // the light sample's shadow ray, or the next bounce
-                shadow_next = (r == STEP_SHADOW);
-                march = route_ray(A, v, *J.scene, slot, ps.org, shadow_next ? ps.shDir : ps.dir);
+                uint32_t set1 = 0;
+                march = route_ray(A, v, *J.scene, slot, ps.org, shadow_next ? ps.shDir : ps.dir, shadow_next,
+                                  word_shobj(job_word(job, ps.shObj)), 0u, 0u, &set1);
+                if (shadow_next)
+                    v.s2[slot] = make_float4(ps.shDir.x, ps.shDir.y, ps.shDir.z, __uint_as_float(set1));
+                again = true;
             }
         }
         push_routed(A, C, nxt, slot, again, march, shadow_next);
@@ -465,6 +482,7 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
     bool active = false, shadow = false;
     uint32_t job = 0, local = 0;
     PathState ps;
+    OriginSignT<float> sign{0.0f, 0u};
     for (;;) {
         // Refill idle lanes from the warp's chunk, claiming chunks as needed,
         // once persist_refill lanes are idle (or none is busy): new samples
@@ -507,6 +525,7 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
                 const CamInfo cam = J.cam;
                 start_sample(ps, ONE ? *S1 : *J.scene, pc, cam, xx, yy, uvx, uvy, (int)k);
                 shadow = false;
+                sign.set = 0u;
                 active = true;
             }
             cbase += n;
@@ -525,7 +544,8 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
             h.materialID = 0.0f;
             h.lightID = -1.0f;
             int objectID = -1;
-            intersect_all<FEAT>(S, ps.org, shadow ? ps.shDir : ps.dir, h, objectID);
+            intersect_all<FEAT>(S, ps.org, shadow ? ps.shDir : ps.dir, h, objectID, shadow, ps.shObj, sign);
+            if (!shadow) sign.set = 0u;  // shading moves the origin
             const StepResult r = shadow ? shade_shadow<false>(ps, S, objectID, depth)
                                         : shade_primary<false>(ps, S, h, objectID, depth);
             shadow = (r == STEP_SHADOW);
