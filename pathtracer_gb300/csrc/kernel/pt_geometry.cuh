@@ -543,28 +543,33 @@ template <typename V, typename R = SOf<V>> PT_DI R sdf(V p) {
 // pt_user_material_d (the FP64 renderer) before including these headers;
 // the precompiled kernels never see that kind.
 //
-// PT_SDF_KINDS (bit k: kind k) lists the kinds a kernel evaluates: a run-time
-// compiled march kernel is given those of the scenes it renders, so the code
-// of the other built-in SDFs is not in it; other kernels take every kind.
+// KINDS (bit k: kind k) lists the kinds a kernel evaluates, PT_SDF_KINDS
+// unless the kernel says so: a run-time compiled march kernel is given those
+// of the scenes it renders, so the code of the other built-in SDFs is not in
+// it, and the built-in march kernels are compiled for classes of kinds; other
+// kernels take every kind.
 #ifndef PT_SDF_KINDS
 #define PT_SDF_KINDS 0xFFFFFFFFu
 #endif
-static_assert(PT_SDF_BLOB == 1 && PT_SDF_MANDELBULB == 2 && PT_SDF_MENGER == 3 && PT_SDF_TERRAIN == 4,
-              "the bit positions tested in plugin_sdf and plugin_material");
-template <typename V, typename R = SOf<V>> PT_DI R plugin_sdf(int kind, int slot, V p) {
+static_assert(PT_SDF_BLOB == 1 && PT_SDF_MANDELBULB == 2,
+              "the bit positions tested in plugin_material");
+template <uint32_t KINDS = PT_SDF_KINDS, typename V, typename R = SOf<V>>
+PT_DI R plugin_sdf(int kind, int slot, V p) {
+    constexpr bool bulb = (KINDS >> PT_SDF_MANDELBULB) & 1u, menger = (KINDS >> PT_SDF_MENGER) & 1u;
+    constexpr bool blob = (KINDS >> PT_SDF_BLOB) & 1u, terrain = (KINDS >> PT_SDF_TERRAIN) & 1u;
     switch (kind) {
-#if (PT_SDF_KINDS >> 2) & 1u
-        case PT_SDF_MANDELBULB: return sdf_mandelbulb::sdf(p);
-#endif
-#if (PT_SDF_KINDS >> 3) & 1u
-        case PT_SDF_MENGER: return sdf_menger::sdf(p);
-#endif
-#if (PT_SDF_KINDS >> 1) & 1u
-        case PT_SDF_BLOB: return sdf_blob::sdf(p);
-#endif
-#if (PT_SDF_KINDS >> 4) & 1u
-        case PT_SDF_TERRAIN: return sdf_terrain::sdf(p);
-#endif
+        case PT_SDF_MANDELBULB:
+            if constexpr (bulb) return sdf_mandelbulb::sdf(p);
+            return R(PT_MAXDIST);
+        case PT_SDF_MENGER:
+            if constexpr (menger) return sdf_menger::sdf(p);
+            return R(PT_MAXDIST);
+        case PT_SDF_BLOB:
+            if constexpr (blob) return sdf_blob::sdf(p);
+            return R(PT_MAXDIST);
+        case PT_SDF_TERRAIN:
+            if constexpr (terrain) return sdf_terrain::sdf(p);
+            return R(PT_MAXDIST);
 #if defined(PT_JIT_USER_SDF)
         case PT_SDF_CUSTOM:
             if constexpr (sizeof(R) == 4) {
@@ -632,13 +637,13 @@ template <typename V, typename R = SOf<V>> PT_DI R scene_sdf(const KScene& S, V 
 // the SDFs they share in the same trip: over each lane's own set, lanes with
 // {0, 1} and lanes with {1} ran SDF 1 in different trips (10.5 of 32 lanes
 // per instruction on menger + terrain).
-template <typename V, typename R = SOf<V>>
+template <uint32_t KINDS = PT_SDF_KINDS, typename V, typename R = SOf<V>>
 PT_DI R scene_sdf_sel(const KScene& S, V p, uint32_t set1, uint32_t walk, int& sel) {
     R sdf = R(PT_MAXDIST);
     sel = -1;
 #if defined(PT_ONE_SDF)
     if (set1 & 1u) {  // as in scene_sdf
-        const R di = plugin_sdf(PT_SDF_CUSTOM, S.meta.custom_base, p - sdf_pos<R>(S, 0));
+        const R di = plugin_sdf<KINDS>(PT_SDF_CUSTOM, S.meta.custom_base, p - sdf_pos<R>(S, 0));
         if (!(sdf < di)) sel = 0;
         sdf = m_fmin(sdf, di);
     }
@@ -651,7 +656,7 @@ PT_DI R scene_sdf_sel(const KScene& S, V p, uint32_t set1, uint32_t walk, int& s
         if (!((bits >> i) & 1u)) continue;
         const int kind = S.plug[i].kind;
         if (kind != PT_SDF_NONE) {
-            const R di = plugin_sdf(kind, S.meta.custom_base + i, p - sdf_pos<R>(S, i));
+            const R di = plugin_sdf<KINDS>(kind, S.meta.custom_base + i, p - sdf_pos<R>(S, i));
             if (!(sdf < di)) sel = i;
             sdf = m_fmin(sdf, di);
         }

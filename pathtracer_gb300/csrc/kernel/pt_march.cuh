@@ -1,6 +1,5 @@
-// pt_march.cuh — the wavefront engine's SDF march kernels (wf_march, and
-// wf_march_warp_normals for dispatches with a mandelbulb) and the helpers
-// every stage kernel shares.  Included by pt_wavefront.cu and, for
+// pt_march.cuh — the wavefront engine's SDF march kernel (wf_march) and the
+// helpers every stage kernel shares.  Included by pt_wavefront.cu and, for
 // scenes whose SDF text is compiled at run time, by the NVRTC program of
 // pt_jit.cu (with PT_JIT_USER_SDF, in namespace ptjit), so both builds run
 // the same source.
@@ -145,66 +144,32 @@ PT_DI uint32_t slot_job(const PoolView& v, uint32_t slot) { return word_job(v.s8
 
 // SphereTracing (SC:779-860) with one SDF evaluation per loop iteration per
 // lane.  A converged ray takes its six normal probes on its own lane
-// (MP_NORMAL0..5), or waits in MP_NORMAL for the warp's normal pass
+// (MP_NORMAL0..5), or leaves the lane for the warp's normal stage
 // (march_rays<true>).
-enum MarchPhase { MP_EMPTY = 0, MP_SIGN = 1, MP_STEP = 2, MP_NORMAL0 = 3, MP_NORMAL5 = 8, MP_NORMAL = 9 };
+enum MarchPhase { MP_EMPTY = 0, MP_SIGN = 1, MP_STEP = 2, MP_NORMAL0 = 3, MP_NORMAL5 = 8, MP_CONVERGED = 9 };
 
-// CalculateNumericalSDFNormals (SC:721-730) for the lanes of `pending` (rays
-// converged at p): the six probes p +- h.xyy, h.yxy, h.yyx of up to five rays
-// at once, one probe per lane, so the probes (near the surface, where an
-// escape-time fractal runs its longest loops) fill the warp instead of one
-// lane each beside rays that march far from it.  Measured on GB300: 11 %
-// less march time on a 12-iteration mandelbulb, 2 % on the 4-iteration one,
-// but 11 % more end to end on menger + terrain, whose evaluations cost the
-// same everywhere and whose probes on the ray's own lane fill the rest of
-// the round.  Returns the
-// central-difference vector (+x - -x, +y - -y, +z - -z) to the lanes of
-// `pending`.  Called by all 32 lanes with the same `pending`.
-PT_DI float3 normal_probes(unsigned pending, const KScene* Sp, float3 p, uint32_t set1, int lane) {
-    const float e = 1e-4f;
-    float3 nv = f3(0.0f, 0.0f, 0.0f);
-    while (pending) {
-        // up to five rays, lowest lanes first (warp-uniform)
-        unsigned take = 0, rest = pending;
-        for (int c = 0; c < 5 && rest; c++) {
-            take |= rest & (0u - rest);
-            rest &= rest - 1u;
-        }
-        const int nray = __popc(take);
-        const int r = lane / 6, j = lane - 6 * r;  // this lane: probe j of the r-th ray taken
-        const bool probe = r < nray;
-        unsigned m = take;  // drop the r lowest rays: the r-th ray is the lowest bit left
-        for (int c = 0; c < r && c < 5; c++) m &= m - 1u;
-        const int src = probe ? __ffs(m) - 1 : lane;
-        const float px = __shfl_sync(0xffffffffu, p.x, src);
-        const float py = __shfl_sync(0xffffffffu, p.y, src);
-        const float pz = __shfl_sync(0xffffffffu, p.z, src);
-        const uint32_t s1 = __shfl_sync(0xffffffffu, set1, src);
-        const uint64_t sp = reinterpret_cast<uint64_t>(Sp);
-        const uint32_t lo = __shfl_sync(0xffffffffu, (uint32_t)sp, src);
-        const uint32_t hi = __shfl_sync(0xffffffffu, (uint32_t)(sp >> 32), src);
-        const uint32_t walk = __reduce_or_sync(0xffffffffu, probe ? s1 : 0u);
-        float val = 0.0f;
-        if (probe) {
-            const KScene& S = *reinterpret_cast<const KScene*>((uint64_t)lo | ((uint64_t)hi << 32));
-            const float ex = (j == 0) ? e : 0.0f, ey = (j == 2) ? e : 0.0f, ez = (j == 4) ? e : 0.0f;
-            const float mx = (j == 1) ? e : 0.0f, my = (j == 3) ? e : 0.0f, mz = (j == 5) ? e : 0.0f;
-            const float3 q = (j & 1) ? f3(px - mx, py - my, pz - mz) : f3(px + ex, py + ey, pz + ez);
-            int esel = -1;
-            val = scene_sdf_sel(S, q, s1, walk, esel);
-        }
-        // Ray lane L collects the probes of its rank among `take`.
-        const int base = 6 * __popc(take & ((1u << lane) - 1u));
-        const float v0 = __shfl_sync(0xffffffffu, val, min(base + 0, 31));
-        const float v1 = __shfl_sync(0xffffffffu, val, min(base + 1, 31));
-        const float v2 = __shfl_sync(0xffffffffu, val, min(base + 2, 31));
-        const float v3 = __shfl_sync(0xffffffffu, val, min(base + 3, 31));
-        const float v4 = __shfl_sync(0xffffffffu, val, min(base + 4, 31));
-        const float v5 = __shfl_sync(0xffffffffu, val, min(base + 5, 31));
-        if ((take >> lane) & 1u) nv = f3(v0 - v1, v2 - v3, v4 - v5);
-        pending &= ~take;
-    }
-    return nv;
+// The normal stage: converged rays whose normal (CalculateNumericalSDFNormals,
+// SC:721-730) and material are still to be taken, per warp.  Sixteen rays'
+// 96 probes are evaluated together, three trips with every lane busy, so
+// near-surface probes (the longest loops of an escape-time fractal) run
+// beside each other and a ray's own lane goes on to its next ray.
+constexpr int kNormalBatch = 16;
+constexpr int kNormalCap = kNormalBatch - 1 + 32;  // fewer than a batch kept, and a round's 32
+struct NormalStage {
+    float4 at[kNormalCap];   // p.xyz, t
+    uint4 of[kNormalCap];    // set1, slot, scene pointer
+    int sel[kNormalCap];     // hit_sel (scene_sdf_material_hit)
+    float probe[6 * kNormalBatch];
+};
+
+// The SDFs a warp's evaluation walks: the union of its lanes' sets
+// (scene_sdf_sel).  Called by all 32 lanes.
+PT_DI uint32_t warp_walk(bool on, uint32_t set1) {
+#if defined(PT_ONE_SDF)
+    return 1u;
+#else
+    return __reduce_or_sync(0xffffffffu, on ? set1 : 0u);
+#endif
 }
 
 // Warp-staged queue appends: lanes with pred add `value` to a per-warp
@@ -241,9 +206,76 @@ PT_DI void stage_flush(const WfArgs& A, uint32_t* buf, uint32_t count, uint32_t*
         queue[b + (uint32_t)lane] = buf[lane];
 }
 
-// The march loop; WARP_NORMALS: normal probes in the warp's pass
-// (normal_probes) instead of on each ray's lane.
-template <bool WARP_NORMALS>
+// Probe j of a hit at p: p +- h.xyy, h.yxy, h.yyx.
+template <typename P> PT_DI float3 probe_point(const P& p, int j) {
+    const float e = 1e-4f;
+    const float ex = (j == 0) ? e : 0.0f, ey = (j == 2) ? e : 0.0f, ez = (j == 4) ? e : 0.0f;
+    const float mx = (j == 1) ? e : 0.0f, my = (j == 3) ? e : 0.0f, mz = (j == 5) ? e : 0.0f;
+    return (j & 1) ? f3(p.x - mx, p.y - my, p.z - mz) : f3(p.x + ex, p.y + ey, p.z + ez);
+}
+
+// The normal stage's evaluation: out of line in run-time compiled kernels,
+// where a second inlined copy of a long snippet cost registers and
+// instruction cache (12-iteration mandelbulb 131.3 against 130.0 ms); inlined
+// it is as fast or faster for the shipped plug-ins.
+#if defined(PT_JIT_USER_SDF)
+template <uint32_t KINDS>
+static __device__ __noinline__ float probe_sdf(const KScene& S, float3 q, uint32_t set1, uint32_t walk) {
+#else
+template <uint32_t KINDS> PT_DI float probe_sdf(const KScene& S, float3 q, uint32_t set1, uint32_t walk) {
+#endif
+    int sel;
+    return scene_sdf_sel<KINDS>(S, q, set1, walk, sel);
+}
+
+// Normals and materials of records [from, from + n), n <= kNormalBatch, into
+// their hit records; returns the record's slot to lane i < n (for the shade
+// queue).  Called by all 32 lanes.
+template <uint32_t KINDS>
+PT_DI uint32_t take_normals(const PoolView& v, NormalStage& ns, int from, int n, int lane) {
+    __syncwarp();
+#pragma unroll 1
+    for (int base = 0; base < 6 * n; base += 32) {
+        const int i = base + lane, r = i / 6, j = i - 6 * r;  // probe j of record r
+        const bool on = i < 6 * n;
+        float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        uint4 b = make_uint4(0u, 0u, 0u, 0u);
+        if (on) {
+            a = ns.at[from + r];
+            b = ns.of[from + r];
+        }
+        const uint32_t walk = warp_walk(on, b.x);
+        if (on) {
+            const KScene& S = *reinterpret_cast<const KScene*>((uint64_t)b.z | ((uint64_t)b.w << 32));
+            const float3 q = probe_point(a, j);
+            ns.probe[i] = probe_sdf<KINDS>(S, q, b.x, walk);
+        }
+    }
+    __syncwarp();
+    uint32_t slot = 0;
+    if (lane < n) {
+        const float* d = ns.probe + 6 * lane;
+        const float4 a = ns.at[from + lane];
+        const uint4 b = ns.of[from + lane];
+        const KScene& S = *reinterpret_cast<const KScene*>((uint64_t)b.z | ((uint64_t)b.w << 32));
+        slot = b.y;
+        const float3 nrm = normalize3(f3(d[0] - d[1], d[2] - d[3], d[4] - d[5]));
+        const float mat = scene_sdf_material_hit(S, f3(a.x, a.y, a.z), b.x, ns.sel[from + lane]);
+        v.h0[slot] = make_float4(a.w - 1e-3f, mat, -1.0f, __int_as_float(-2));
+        v.h1[slot] = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
+    }
+    __syncwarp();  // the records may be overwritten from here on
+    return slot;
+}
+
+// The march loop over the SDF plug-ins KINDS (bit k: kind k).  STAGED: normals
+// in the warp's normal stage; otherwise on each ray's lane, where the probes
+// fill the rest of the round: better where every evaluation costs about the
+// same.  Measured on GB300 with the scene's kinds: menger + terrain 1080p 16
+// spp on the lane 93.9 ms, staged 103.5; against probing at the end of every
+// round, up to five rays a pass: 12-iteration mandelbulb 1024x1024x64 staged
+// 130.0 ms, 132.4 so; shipped mandelbulb 777x431x16 11.4 ms, 11.7 so.
+template <bool STAGED, uint32_t KINDS>
 PT_DI void march_rays(const WfArgs& A) {
     WfCounters& C = *A.counters;
     const uint32_t cur = C.cur;
@@ -266,6 +298,8 @@ PT_DI void march_rays(const WfArgs& A) {
     // queues 32 at a time.
     __shared__ uint32_t staged[kStageThreads / 32][2][64];
     uint32_t nstaged[2] = {0u, 0u};  // warp-uniform: primary hits, shadow results
+    __shared__ NormalStage normals[STAGED ? kStageThreads / 32 : 1];
+    int nnormals = 0;  // warp-uniform: records in the warp's normal stage
     const int wib = (int)(threadIdx.x >> 5);
 
     uint32_t slot = 0;
@@ -274,14 +308,14 @@ PT_DI void march_rays(const WfArgs& A) {
     bool exhausted = false;
     float3 org = f3(0.0f, 0.0f, 0.0f), dir = f3(0.0f, 0.0f, 1.0f), p = org;
     float t = 0.0f, insT = 0.0f, omega = 0.0f, prevR = 0.0f, hitdist = 0.0f, k = 0.0f, nplus = 0.0f;
-    float3 nv = f3(0.0f, 0.0f, 0.0f);
+    float3 nv = f3(0.0f, 0.0f, 0.0f);  // nplus, nv: normals on the ray's lane only
     float2 tmm = make_float2(0.0f, 0.0f);
     uint32_t set1 = 0;
     int points = 0, iter = 0;
     bool xmarch = false;  // the ray's scene sets march limits (PT_EXT_MARCH; read from it where used)
     int hit_sel = -2;  // >= -1 once the lane's march converged (scene_sdf_material_hit)
     bool shadow_ray = false;
-    const float omegaMax = kOmegaMax, omegaSpeed = 0.20f, e = 1e-4f;
+    const float omegaMax = kOmegaMax, omegaSpeed = 0.20f;
 
     for (;;) {
         // Refill lanes that have no ray (warp-aggregated fetch), once at
@@ -363,26 +397,16 @@ PT_DI void march_rays(const WfArgs& A) {
             if (sub > 0 && __ballot_sync(0xffffffffu, evalLane) == 0) break;
             float3 q = p;
             if (phase == MP_SIGN) q = org;
-            if (!WARP_NORMALS && phase >= MP_NORMAL0 && phase <= MP_NORMAL5) {
-                // CalculateNumericalSDFNormals (SC:721-730): p +- h.xyy, h.yxy, h.yyx
-                const int j = phase - MP_NORMAL0;
-                const float ex = (j == 0) ? e : 0.0f, ey = (j == 2) ? e : 0.0f, ez = (j == 4) ? e : 0.0f;
-                const float mx = (j == 1) ? e : 0.0f, my = (j == 3) ? e : 0.0f, mz = (j == 5) ? e : 0.0f;
-                q = (j & 1) ? f3(p.x - mx, p.y - my, p.z - mz) : f3(p.x + ex, p.y + ey, p.z + ez);
-            }
+            if (!STAGED && phase >= MP_NORMAL0 && phase <= MP_NORMAL5) q = probe_point(p, phase - MP_NORMAL0);
             float val = 0.0f;
             int esel = -1;
-#if defined(PT_ONE_SDF)
-            const uint32_t walk = 1u;
-#else
-            const uint32_t walk = __reduce_or_sync(0xffffffffu, evalLane ? set1 : 0u);
-#endif
-            if (evalLane) val = scene_sdf_sel(*Sp, q, set1, walk, esel);
+            const uint32_t walk = warp_walk(evalLane, set1);
+            if (evalLane) val = scene_sdf_sel<KINDS>(*Sp, q, set1, walk, esel);
             if (!evalLane) continue;
             if (phase == MP_SIGN) {
                 k = sign_glsl(val);
                 phase = MP_STEP;
-            } else if (phase == MP_STEP) {
+            } else if (STAGED || phase == MP_STEP) {
                 const float radius = val;
                 bool exitLoop = false;
                 if (xmarch && t > Sp->ext.march_max_distance) {
@@ -436,7 +460,7 @@ PT_DI void march_rays(const WfArgs& A) {
                         finished = true;
                     } else if (t < hitdist) {
                         p = fma3s(dir, t, org);
-                        phase = WARP_NORMALS ? MP_NORMAL : MP_NORMAL0;
+                        phase = STAGED ? MP_CONVERGED : MP_NORMAL0;
                     } else {
                         finished = true;
                     }
@@ -447,7 +471,7 @@ PT_DI void march_rays(const WfArgs& A) {
                                              __uint_as_float(set1));
                     suspend = true;
                 }
-            } else if (!WARP_NORMALS && phase >= MP_NORMAL0 && phase <= MP_NORMAL5) {
+            } else if (!STAGED) {
                 const int j = phase - MP_NORMAL0;
                 if ((j & 1) == 0) {
                     nplus = val;
@@ -465,19 +489,26 @@ PT_DI void march_rays(const WfArgs& A) {
             }
         }
 
-        if constexpr (WARP_NORMALS) {
-            // The normals of this round's converged rays, six probes a ray
-            // across the warp.
-            const unsigned pending = __ballot_sync(0xffffffffu, phase == MP_NORMAL);
-            if (pending) {
-                const float3 nw = normal_probes(pending, Sp, p, set1, lane);
-                if (phase == MP_NORMAL) {
-                    hit = true;
-                    finished = true;
-                    const float3 nrm = normalize3(nw);
-                    const float mat = scene_sdf_material_hit(*Sp, p, set1, hit_sel);
-                    v.h0[slot] = make_float4(t - 1e-3f, mat, -1.0f, __int_as_float(-2));
-                    v.h1[slot] = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
+        if constexpr (STAGED) {
+            // Converged rays give their lanes up; a full batch of them takes
+            // its normals.
+            const unsigned conv = __ballot_sync(0xffffffffu, phase == MP_CONVERGED);
+            if (conv) {
+                NormalStage& ns = normals[wib];
+                if (phase == MP_CONVERGED) {
+                    const int at = nnormals + __popc(conv & ((1u << lane) - 1u));
+                    const uint64_t sp = reinterpret_cast<uint64_t>(Sp);
+                    ns.at[at] = make_float4(p.x, p.y, p.z, t);
+                    ns.of[at] = make_uint4(set1, slot, (uint32_t)sp, (uint32_t)(sp >> 32));
+                    ns.sel[at] = hit_sel;
+                    phase = MP_EMPTY;
+                }
+                nnormals += __popc(conv);
+                while (nnormals >= kNormalBatch) {
+                    nnormals -= kNormalBatch;
+                    const uint32_t ready = take_normals<KINDS>(v, ns, nnormals, kNormalBatch, lane);
+                    stage_push(A, staged[wib][0], nstaged[0], lane < kNormalBatch, ready, A.q_shade[cur], &C.n_shade[cur],
+                               lane);
                 }
             }
         } else if (finished && hit && !shadow_ray) {
@@ -494,20 +525,28 @@ PT_DI void march_rays(const WfArgs& A) {
         if (finished || suspend) phase = MP_EMPTY;
     }
     // The staged remainders.
+    if (STAGED && nnormals) {
+        const uint32_t ready = take_normals<KINDS>(v, normals[wib], 0, nnormals, lane);
+        stage_push(A, staged[wib][0], nstaged[0], lane < nnormals, ready, A.q_shade[cur], &C.n_shade[cur], lane);
+    }
     stage_flush(A, staged[wib][0], nstaged[0], A.q_shade[cur], &C.n_shade[cur], lane);
     stage_flush(A, staged[wib][1], nstaged[1], A.q_shadow[cur], &C.n_shadow[cur], lane);
 }
 
+// The run-time compiled kernel holds its scenes' kinds (PT_SDF_KINDS); the
+// built-in ones are compiled for every kind, for the mandelbulb alone and
+// for the kinds without it, whose evaluations cost the same everywhere: the
+// host picks the smallest that covers a dispatch.  Code of kinds that a
+// scene does not have cost menger + terrain 10 % and the shipped mandelbulb
+// 2 % (instruction cache, registers).
 #if defined(PT_JIT_USER_SDF)
-// Run-time compiled snippets: the warp's normal pass (escape-time fractals
-// are the usual reason to write one, and their cost is not known here).
-__global__ void PT_MARCH_BOUNDS wf_march(const __grid_constant__ WfArgs A) { march_rays<true>(A); }
+__global__ void PT_MARCH_BOUNDS wf_march(const __grid_constant__ WfArgs A) { march_rays<true, PT_SDF_KINDS>(A); }
 #else
-// The shipped plug-ins: normals on each ray's lane (menger, terrain and blob
-// cost the same everywhere), or in the warp's pass when a mandelbulb is in
-// the dispatch (the host picks the kernel).
-__global__ void PT_MARCH_BOUNDS wf_march(const __grid_constant__ WfArgs A) { march_rays<false>(A); }
-__global__ void PT_MARCH_BOUNDS wf_march_warp_normals(const __grid_constant__ WfArgs A) { march_rays<true>(A); }
+constexpr uint32_t kKindsBulb = 1u << PT_SDF_MANDELBULB;
+constexpr uint32_t kKindsEven = (1u << PT_SDF_BLOB) | (1u << PT_SDF_MENGER) | (1u << PT_SDF_TERRAIN);
+__global__ void PT_MARCH_BOUNDS wf_march(const __grid_constant__ WfArgs A) { march_rays<true, 0xFFFFFFFFu>(A); }
+__global__ void PT_MARCH_BOUNDS wf_march_bulb(const __grid_constant__ WfArgs A) { march_rays<true, kKindsBulb>(A); }
+__global__ void PT_MARCH_BOUNDS wf_march_even(const __grid_constant__ WfArgs A) { march_rays<false, kKindsEven>(A); }
 #endif
 
 }  // namespace

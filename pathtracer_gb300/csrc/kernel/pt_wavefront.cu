@@ -659,8 +659,11 @@ static int resident_blocks(const void* kernel, int* cache) {
     return *cache;
 }
 
-const void* PTK_WF(ptk_wavefront_march_warp_normals)() {
-    return reinterpret_cast<const void*>(wf_march_warp_normals);
+const void* PTK_WF(ptk_wavefront_march)(uint32_t kinds) {
+    kinds &= ~(1u << PT_SDF_NONE);
+    if ((kinds & ~kKindsEven) == 0) return reinterpret_cast<const void*>(wf_march_even);
+    if ((kinds & ~kKindsBulb) == 0) return reinterpret_cast<const void*>(wf_march_bulb);
+    return reinterpret_cast<const void*>(wf_march);
 }
 
 cudaError_t PTK_WF(ptk_wavefront_launch_iteration)(const WfArgs* a, bool trace, int grid, cudaStream_t stream,
@@ -755,7 +758,7 @@ cudaError_t PTK_WF(ptk_wavefront_launch_resolve)(const WfArgs* a, uint32_t job, 
 extern const WfKernelSet PTK_WF(ptk_wavefront_kernel_set);
 const WfKernelSet PTK_WF(ptk_wavefront_kernel_set) = {
     PTK_WF(ptk_wavefront_launch_init),        PTK_WF(ptk_wavefront_launch_job_add),
-    PTK_WF(ptk_wavefront_launch_iteration),   PTK_WF(ptk_wavefront_march_warp_normals),
+    PTK_WF(ptk_wavefront_launch_iteration),   PTK_WF(ptk_wavefront_march),
     PTK_WF(ptk_persist_launch),               PTK_WF(ptk_persist_blocks_per_sm),
     PTK_WF(ptk_wavefront_launch_resolve),
 };

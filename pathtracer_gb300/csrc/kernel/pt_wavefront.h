@@ -114,15 +114,14 @@ cudaError_t ptk_wavefront_launch_job_add(const WfArgs* a, const WfJob* job, uint
 // One iteration: march, shade, gen, bookkeeping (grid = blocks per stage
 // kernel, capped per kernel at what is resident); with stage_events, 6
 // events bracket the 5 stages (isect, done inside shade and gen, stays empty).
-// march_kernel: the march kernel to launch instead of the built-in wf_march:
-// a run-time compiled one (pt_jit.cu; scenes with SDF snippets compiled at
-// run time) or ptk_wavefront_march_warp_normals().
+// march_kernel: the march kernel to launch: a run-time compiled one (pt_jit.cu;
+// scenes with SDF snippets compiled at run time) or one of
+// ptk_wavefront_march's; null: the built-in one for every kind.
 cudaError_t ptk_wavefront_launch_iteration(const WfArgs* a, bool trace, int grid, cudaStream_t stream,
                                            cudaEvent_t* stage_events = nullptr, const void* march_kernel = nullptr);
-// The built-in march kernel that probes normals across the warp, for
-// dispatches with a mandelbulb (pass it as march_kernel; the default
-// built-in kernel probes each ray's normal on its own lane).
-const void* ptk_wavefront_march_warp_normals();
+// The built-in march kernel for scenes with SDF plug-ins `kinds` (bit k: kind
+// k; bit 0, slots without a plug-in, is ignored).
+const void* ptk_wavefront_march(uint32_t kinds);
 // Kernels launched per staged iteration (march, shade, gen, bookkeeping).
 constexpr int kWfKernelsPerIteration = 4;
 // Stages timed by the engine's stage-timing mode.
@@ -148,7 +147,7 @@ struct WfKernelSet {
     cudaError_t (*init)(const WfArgs*, cudaStream_t);
     cudaError_t (*job_add)(const WfArgs*, const WfJob*, uint32_t, uint32_t, cudaStream_t);
     cudaError_t (*iteration)(const WfArgs*, bool, int, cudaStream_t, cudaEvent_t*, const void*);
-    const void* (*march_warp_normals)();
+    const void* (*march)(uint32_t kinds);
     cudaError_t (*persist)(const WfArgs*, int, int, uint64_t, const KScene*, cudaStream_t);
     int (*persist_blocks_per_sm)(int);
     cudaError_t (*resolve)(const WfArgs*, uint32_t, const pt_push*, float4*, const float4*, cudaStream_t);

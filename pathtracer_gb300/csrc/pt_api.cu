@@ -696,10 +696,9 @@ static int dispatch_wavefront(pt_ctx* ctx, const pt_push* push) {
     for (int e = 0; e < kMax; e++)
         if (*slot[e]) launches0 += (*slot[e])->kernel_launches;
     // Run-time compiled SDF snippets: their march kernel (the other stages
-    // evaluate no SDF); a mandelbulb: the built-in kernel with the warp-wide
-    // normal pass.
-    bool bulb = false;
-    for (int i = 0; i < ctx->nplug; i++) bulb = bulb || ctx->plug[i].kind == PT_SDF_MANDELBULB;
+    // evaluate no SDF); else the built-in one for the scene's kinds.
+    uint32_t kinds = 0;
+    for (int i = 0; i < ctx->nplug; i++) kinds |= 1u << ctx->plug[i].kind;
     for (int e = 0; e < n; e++) {
         const uint32_t share = base[e + 1] - base[e];
         uint32_t pool = share < ctx->pool_cap ? share : ctx->pool_cap;
@@ -715,7 +714,7 @@ static int dispatch_wavefront(pt_ctx* ctx, const pt_push* push) {
         W->set_march_kernel(!ctx->custom.empty()
                                 ? reinterpret_cast<const void*>(
                                       ctx->jit[kJitMarch][(size_t)ctx->jit_cur[kJitMarch]].kernel[0])
-                                : (bulb ? W->kernels->march_warp_normals() : nullptr));
+                                : W->kernels->march(kinds));
     }
     const size_t cbytes = (size_t)total * sizeof(float4);
     if (cbytes > ctx->colors_bytes) {

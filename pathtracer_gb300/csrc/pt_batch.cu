@@ -135,9 +135,6 @@ struct pt_batch {
     uint32_t sdf_kinds = 0;  // plug-in kinds of every scene added (bit k: kind k)
     uint32_t jit_kinds = 0;  // the kinds `jit` was compiled for (PT_SDF_KINDS)
     JitModule jit64;  // the FP64 renderer's megakernel for the same snippets (pt_batch_render_fp64), when needed
-    // A scene with a mandelbulb was added: the staged engine's built-in march
-    // kernel then probes normals across the warp.
-    bool bulb = false;
     std::string err;
 };
 
@@ -171,11 +168,10 @@ BatchPass* pass_at(pt_batch* b, uint32_t j) {
 }
 
 // The staged engine's march kernel: the batch's run-time compiled one, else
-// the built-in one with the warp-wide normal pass when a mandelbulb is in
-// the batch, else the default built-in one (null).
+// the built-in one for the kinds of every scene added.
 const void* staged_march_kernel(const pt_batch* b) {
-    if (b->jit.lib) return reinterpret_cast<const void*>(b->jit.kernel[0]);
-    return b->bulb ? ptk_wavefront_kernels(b->device_checks)->march_warp_normals() : nullptr;
+    return b->jit.lib ? reinterpret_cast<const void*>(b->jit.kernel[0])
+                      : ptk_wavefront_kernels(b->device_checks)->march(b->sdf_kinds);
 }
 
 // Creates engine e on first use: a staged engine with the batch's pool,
@@ -476,13 +472,12 @@ int add_scene(pt_batch* b, const pt_ubo* ubo, const pt_sdf_plugin* plugins, int 
         return bfail(b, PT_ERR_INVALID, "pt_batch_add_scene: objects overflow the 1024-float object array");
     if (n[5] > PT_MAX_LIVE_SDFS || nplugins > PT_MAX_LIVE_SDFS)
         return bfail(b, PT_ERR_UNSUPPORTED, "pt_batch_add_scene: at most 32 SDFs can be evaluated (32-bit set mask)");
-    bool custom = false, bulb = false;
+    bool custom = false;
     uint32_t kinds = 0;
     for (int i = 0; i < nplugins; i++) {
         if (plugins[i].kind < PT_SDF_NONE || plugins[i].kind > PT_SDF_CUSTOM)
             return bfail(b, PT_ERR_INVALID, "pt_batch_add_scene: unknown plug-in kind");
         custom = custom || plugins[i].kind == PT_SDF_CUSTOM;
-        bulb = bulb || plugins[i].kind == PT_SDF_MANDELBULB;
         kinds |= 1u << plugins[i].kind;
     }
     PT_B_TRY(b, cudaSetDevice(b->device));
@@ -531,7 +526,6 @@ int add_scene(pt_batch* b, const pt_ubo* ubo, const pt_sdf_plugin* plugins, int 
     bs.has_sdf = n[5] > 0;
     bs.custom = custom;
     bs.variant = pt_feature_variant(n);
-    b->bulb = b->bulb || bulb;
     // the compiled march kernel holds the code of the kinds seen so far: a
     // scene with another kind needs it compiled again
     b->sdf_kinds |= kinds;
@@ -766,7 +760,7 @@ int pt_batch_step(pt_batch* b, int iterations, int* completed, int capacity, int
     if (jr != PT_OK) return jr;
     for (int se : {kStaged, kStaged2})
         if (b->engine_live[se] && b->engine[se].march_kernel != staged_march_kernel(b)) {
-            // a mandelbulb scene arrived: no launch of the old kernel may be in flight
+            // a scene of another kind arrived: no launch of the old kernel may be in flight
             PT_B_TRY(b, cudaStreamSynchronize(b->estream[se]));
             b->engine[se].set_march_kernel(staged_march_kernel(b));
         }

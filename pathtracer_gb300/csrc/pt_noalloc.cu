@@ -172,10 +172,9 @@ extern "C" int pt_dispatch_noalloc(const pt_ubo* ubo, const pt_sdf_plugin* plugi
     WfJob job_table[1];
     PT_NA_TRY(engine.attach(device, stream, total < kPool ? (total < 1024u ? 1024u : total) : kPool, 1, 64,
                             base + kEngineOff, kEngineBytes, &counters, job_table));
-    // A mandelbulb marches with the warp-wide normal pass, as pt_dispatch does.
-    bool bulb = false;
-    for (int i = 0; i < nplugins; i++) bulb = bulb || plugins[i].kind == PT_SDF_MANDELBULB;
-    engine.set_march_kernel(bulb ? ptk_wavefront_march_warp_normals() : nullptr);
+    uint32_t kinds = 0;
+    for (int i = 0; i < nplugins; i++) kinds |= 1u << plugins[i].kind;
+    engine.set_march_kernel(ptk_wavefront_march(kinds));
     WfJob j;
     std::memset(&j, 0, sizeof j);
     j.scene = d_scene;
