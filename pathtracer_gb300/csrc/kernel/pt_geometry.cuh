@@ -42,9 +42,11 @@ template <typename V> PT_DI bool bounding_sphere(V org, V dir, V pos, ND<SOf<V>>
     return true;
 }
 
-// SphereIntersection, SC:289-317.
-template <typename R>
-PT_DI bool sphere_intersect(V3<R> org, V3<R> dir, V3<R> pos, ND<R> radius, ND<R> mat, ND<R> light, HitT<R>& h) {
+// SphereIntersection, SC:289-317, up to the accepted distance: t and the side
+// when the sphere is hit nearer than `nearest`.  The hit's normal follows
+// from them (sphere_normal), once the nearest object is known.
+template <typename V, typename R = SOf<V>>
+PT_DI bool sphere_hit(V org, V dir, V pos, ND<R> radius, R& nearest, bool& outside) {
     const V3<R> lo = org - pos;
     const R b = R(2) * dot3(dir, lo);
     const R c = dot3(lo, lo) - (radius * radius);
@@ -54,16 +56,83 @@ PT_DI bool sphere_intersect(V3<R> org, V3<R> dir, V3<R> pos, ND<R> radius, ND<R>
     const R t1 = (-b - sqrtD) * R(0.5);
     const R t2 = (-b + sqrtD) * R(0.5);
     const R t = (t1 > R(0)) ? t1 : t2;
-    const R isOutside = (t1 > R(0)) ? R(1) : R(-1);
     if (t < PT_LIT(R, 1e-4)) return false;
-    if (t < h.hitdist) {
-        h.hitdist = t;
-        h.normal = normalize3(fma3s(dir, t, lo) * isOutside);
-        h.materialID = mat;
-        h.lightID = light;
+    if (t < nearest) {
+        nearest = t;
+        outside = t1 > R(0);
         return true;
     }
     return false;
+}
+template <typename V, typename R = SOf<V>> PT_DI V sphere_normal(V org, V dir, V pos, ND<R> t, bool outside) {
+    return normalize3(fma3s(dir, t, org - pos) * (outside ? R(1) : R(-1)));
+}
+
+// The sphere loop: the nearest sphere below h.hitdist, in object order;
+// returns its index (-1 for none) and leaves its distance in h.hitdist.
+// `objs`: the scene's object floats where lanes can read different spheres
+// at once (shared or global memory; the constant bank serves one address at
+// a time).
+//
+// Most spheres are missed, and each test runs as long as the warp's slowest
+// lane: with 34 spheres some lane passes the discriminant of almost every
+// one and the whole warp takes its square root and normal (2,800 instructions
+// a ray and step).  So a first pass bounds the discriminant from hoisted
+// dot products, d.(o - p) = d.o - d.p and |o - p|^2 - r^2 = |o|^2 - 2 o.p +
+// (|p|^2 - r^2), eight fused operations a sphere, and collects the spheres
+// that may be hit; then each lane tests its own few exactly.  A sphere is
+// left out only when the exact test is sure to refuse it:
+// - its discriminant is negative by the margin: with u = 2^-24 the exact
+//   test's rounding moves b^2/4 - c by at most 15 u |o-p|^2 + 3 u r^2, the
+//   bound's by at most 42 u (|o|^2 + |p|^2) + 9 u r^2, and the double
+//   renderer's narrowing of o and d by 24 u (|o|^2 + |p|^2): together below
+//   100 u (|o|^2 + |p|^2 + r^2), against a margin of 256 u;
+// - or the origin is outside (c > 0 by the margin) and the ray leaves
+//   (d.(o-p) above its error 12 u (|o| + |p|)): then fl(b^2 - 4c) <= fl(b^2),
+//   its root is at most b and both distances are <= 0.
+// NaN and infinities fail both comparisons or cannot hit.  From four spheres
+// on; below, the pass costs what it saves.
+constexpr int kCullMin = 4;
+template <typename R>
+PT_DI int intersect_spheres(const KScene& S, const float* __restrict__ objs, V3<R> org, V3<R> dir, R& nearest,
+                            bool& outside) {
+    const int n0 = S.meta.n[0];
+    int win = -1;
+    if (n0 < kCullMin) {
+#pragma unroll 1
+        for (int i = 0; i < n0; i++) {
+            const float* o = S.objects + 6 * i;
+            if (sphere_hit(org, dir, v3<R>(o[0], o[1], o[2]), o[3], nearest, outside)) win = i;
+        }
+        return win;
+    }
+    const float ox = (float)org.x, oy = (float)org.y, oz = (float)org.z;
+    const float dx = (float)dir.x, dy = (float)dir.y, dz = (float)dir.z;
+    const float oo = __fmaf_rn(ox, ox, __fmaf_rn(oy, oy, oz * oz));
+    const float od = __fmaf_rn(ox, dx, __fmaf_rn(oy, dy, oz * dz));
+    const float ook = oo * (float)(1.0 - PT_CULL_EPS);
+    const float ox2 = -2.0f * ox, oy2 = -2.0f * oy, oz2 = -2.0f * oz;
+    const float leaving = 3.814697265625e-06f * (0.5f + 0.5f * oo + S.cull_pmax);  // 2^-18: 64 u (|o| + |p|)
+#pragma unroll 1
+    for (int base = 0; base < n0; base += 32) {
+        uint32_t may = 0;
+        const int cnt = min(32, n0 - base);
+#pragma unroll 4
+        for (int j = 0; j < cnt; j++) {
+            const float4 s = S.cull[base + j];
+            const float hb = __fmaf_rn(-dx, s.x, __fmaf_rn(-dy, s.y, __fmaf_rn(-dz, s.z, od)));
+            const float c = __fmaf_rn(ox2, s.x, __fmaf_rn(oy2, s.y, __fmaf_rn(oz2, s.z, ook + s.w)));
+            const bool miss = (__fmaf_rn(hb, hb, -c) < 0.0f) || (hb > leaving && c > 0.0f);
+            may |= miss ? 0u : (1u << j);
+        }
+        while (may) {
+            const int i = base + __ffs(may) - 1;
+            may &= may - 1u;
+            const float* o = objs + 6 * i;
+            if (sphere_hit(org, dir, v3<R>(o[0], o[1], o[2]), o[3], nearest, outside)) win = i;
+        }
+    }
+    return win;
 }
 
 // PlaneIntersection, SC:319-335.
@@ -83,10 +152,10 @@ PT_DI bool plane_intersect(V3<R> org, V3<R> dir, V3<R> pos, ND<R> mat, ND<R> lig
     return false;
 }
 
-// BoxIntersection, SC:337-364 (matrix from KScene::rot).
-template <typename R>
-PT_DI bool box_intersect(V3<R> org, V3<R> dir_w, V3<R> pos, V3<R> size, const M3<R>& m, ND<R> mat, ND<R> light,
-                         HitT<R>& h) {
+// BoxIntersection, SC:337-364 (matrix from KScene::rot), up to the accepted
+// distance; the normal follows from it (box_normal).
+template <typename V, typename R = SOf<V>>
+PT_DI bool box_hit(V org, V dir_w, V pos, V size, const M3<R>& m, R& nearest) {
     const V3<R> lo = mul_vm(org - pos, m);
     const V3<R> dir = mul_vm(dir_w, m);
     const V3<R> invdir = v3<R>(R(1) / dir.x, R(1) / dir.y, R(1) / dir.z);
@@ -97,18 +166,21 @@ PT_DI bool box_intersect(V3<R> org, V3<R> dir_w, V3<R> pos, V3<R> size, const M3
     const R t2 = m_fmin(m_fmin(bb.x, bb.y), bb.z);
     const R t = (t1 < R(0)) ? t2 : t1;
     if ((t1 > t2) || (t < PT_LIT(R, 1e-4))) return false;
-    if (t < h.hitdist) {
-        h.hitdist = t;
-        const V3<R> p = abs3((lo + dir * t) / size);
-        const R mx = m_fmax(m_fmax(p.x, p.y), p.z);
-        const V3<R> st = v3<R>(step_glsl(mx, p.x), step_glsl(mx, p.y), step_glsl(mx, p.z));
-        const V3<R> sg = v3<R>(-sign_glsl(dir.x), -sign_glsl(dir.y), -sign_glsl(dir.z));
-        h.normal = mul_mv(m, st * sg);
-        h.materialID = mat;
-        h.lightID = light;
+    if (t < nearest) {
+        nearest = t;
         return true;
     }
     return false;
+}
+template <typename V, typename R = SOf<V>>
+PT_DI V box_normal(V org, V dir_w, V pos, V size, const M3<R>& m, ND<R> t) {
+    const V3<R> lo = mul_vm(org - pos, m);
+    const V3<R> dir = mul_vm(dir_w, m);
+    const V3<R> p = abs3((lo + dir * t) / size);
+    const R mx = m_fmax(m_fmax(p.x, p.y), p.z);
+    const V3<R> st = v3<R>(step_glsl(mx, p.x), step_glsl(mx, p.y), step_glsl(mx, p.z));
+    const V3<R> sg = v3<R>(-sign_glsl(dir.x), -sign_glsl(dir.y), -sign_glsl(dir.z));
+    return mul_mv(m, st * sg);
 }
 
 // Lens geometry shared by the camera lens and scene lenses.
@@ -177,7 +249,7 @@ PT_DI bool lens_intersect(V3<R> org, V3<R> dir, const LensGeomT<R>& L, ND<R> mat
     if (L.converging) lensSlicePos += lensThicknessHalf;
     const R sliceRadius = R(2) * L.focal;
     bool hit = false;
-#pragma unroll
+#pragma unroll 1
     for (int i = 0; i < 2; i++) {
         if (slice_intersect(org, dir, L, sliceRadius, lensThicknessHalf, i == 0, lensSlicePos, !L.converging, mat,
                             light, h, isOutside))
@@ -858,20 +930,17 @@ PT_DI bool sphere_trace(const KScene& S, V3<R> org, V3<R> dir, HitT<R>& h, bool 
 
 // The analytic part of Intersection (SC:862-923) and of the object loop of
 // LightSourceVisibilityCheck (SC:1121-1201): objectID = index of the last
-// object whose test hit, -1 for none.
+// object whose test hit, -1 for none.  Spheres and boxes leave their normal
+// and ids to the end, for the one that is nearest; a shadow ray, of which
+// only objectID (and hitdist, for a march) is read, takes neither.  objs:
+// see intersect_spheres.
 template <int FEAT = PT_FEAT_ALL, typename R = float>
-PT_DI void intersect_analytic(const KScene& S, V3<R> org, V3<R> dir, HitT<R>& h, int& objectID) {
-    int id = -1;
+PT_DI void intersect_analytic(const KScene& S, const float* __restrict__ objs, V3<R> org, V3<R> dir, HitT<R>& h,
+                              int& objectID, bool shadow) {
     const int n0 = S.meta.n[0], n1 = S.meta.n[1], n2 = S.meta.n[2], n3 = S.meta.n[3], n4 = S.meta.n[4];
-    int gi = 0;
-#pragma unroll 1
-    for (int i = 0; i < n0; i++, gi++) {
-        const int b = 6 * i;
-        const V3<R> pos = v3<R>(S.objects[b], S.objects[b + 1], S.objects[b + 2]);
-        if (sphere_intersect(org, dir, pos, S.objects[b + 3], (R)((int)S.objects[b + 4] - 1),
-                             (R)((int)S.objects[b + 5] - 1), h))
-            id = gi;
-    }
+    bool outside = false;
+    int id = intersect_spheres<R>(S, objs, org, dir, h.hitdist, outside);
+    int gi = n0;
 #pragma unroll 1
     for (int i = 0; i < n1; i++, gi++) {
         const int b = S.meta.offset[1] + 5 * i;
@@ -887,9 +956,7 @@ PT_DI void intersect_analytic(const KScene& S, V3<R> org, V3<R> dir, HitT<R>& h,
             const V3<R> pos = v3<R>(S.objects[b], S.objects[b + 1], S.objects[b + 2]);
             const V3<R> size = v3<R>(S.objects[b + 6], S.objects[b + 7], S.objects[b + 8]);
             if (!bounding_sphere(org, dir, pos, PT_LIT(R, 0.25) * dot3(size, size))) continue;
-            if (box_intersect(org, dir, pos, size, s_rotation_r<R>(S, gi), (R)((int)S.objects[b + 9] - 1),
-                              (R)((int)S.objects[b + 10] - 1), h))
-                id = gi;
+            if (box_hit(org, dir, pos, size, s_rotation_r<R>(S, gi), h.hitdist)) id = gi;
         }
     }
     if constexpr ((FEAT & PT_FEAT_LENS) != 0) {
@@ -921,6 +988,21 @@ PT_DI void intersect_analytic(const KScene& S, V3<R> org, V3<R> dir, HitT<R>& h,
         }
     }
     objectID = id;
+    if (shadow || id < 0) return;
+    const int box0 = n0 + n1;
+    if (id < n0) {
+        const float* o = objs + 6 * id;
+        h.normal = sphere_normal(org, dir, v3<R>(o[0], o[1], o[2]), h.hitdist, outside);
+        h.materialID = (R)((int)o[4] - 1);
+        h.lightID = (R)((int)o[5] - 1);
+    } else if ((FEAT & PT_FEAT_BOX) != 0 && id >= box0 && id < box0 + n2) {
+        const int b = S.meta.offset[2] + 11 * (id - box0);
+        const V3<R> pos = v3<R>(S.objects[b], S.objects[b + 1], S.objects[b + 2]);
+        const V3<R> size = v3<R>(S.objects[b + 6], S.objects[b + 7], S.objects[b + 8]);
+        h.normal = box_normal(org, dir, pos, size, s_rotation_r<R>(S, id), h.hitdist);
+        h.materialID = (R)((int)S.objects[b + 9] - 1);
+        h.lightID = (R)((int)S.objects[b + 10] - 1);
+    }
 }
 
 // Intersection (SC:862-934) / LightSourceVisibilityCheck's loop: the analytic
@@ -930,9 +1012,9 @@ PT_DI void intersect_analytic(const KScene& S, V3<R> org, V3<R> dir, HitT<R>& h,
 // was reached.  `sign`: see OriginSignT; the caller clears its set whenever
 // the path's origin moves.
 template <int FEAT = PT_FEAT_ALL, typename R = float>
-PT_DI void intersect_all(const KScene& S, V3<R> org, V3<R> dir, HitT<R>& h, int& objectID, bool shadow, int shObj,
-                         OriginSignT<R>& sign) {
-    intersect_analytic<FEAT>(S, org, dir, h, objectID);
+PT_DI void intersect_all(const KScene& S, const float* __restrict__ objs, V3<R> org, V3<R> dir, HitT<R>& h,
+                         int& objectID, bool shadow, int shObj, OriginSignT<R>& sign) {
+    intersect_analytic<FEAT>(S, objs, org, dir, h, objectID, shadow);
     if constexpr ((FEAT & PT_FEAT_SDF) != 0) {
         if (S.meta.n[5] > 0 && !(shadow && !shadow_needs_march(objectID, shObj))) {
             if (sphere_trace(S, org, dir, h, shadow, sign)) objectID = -2;

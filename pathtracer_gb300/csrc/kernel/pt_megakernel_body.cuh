@@ -34,6 +34,9 @@ __global__ void __launch_bounds__(PT_MK_THREADS) megakernel(const __grid_constan
     const pt_push& pc = P.pc;
     __shared__ CamInfoT<R> camS;
     if (threadIdx.x == 0 && threadIdx.y == 0) camS = make_camera<R>(pc);
+    // the spheres, where lanes can read different ones at once
+    __shared__ float sphS[6 * PT_MAX_SCENE_SPHERES];
+    for (int i = threadIdx.y * blockDim.x + threadIdx.x; i < 6 * S.meta.n[0]; i += PT_MK_THREADS) sphS[i] = S.objects[i];
     __syncthreads();
 
     const int W = pc.resolution[0], H = pc.resolution[1];
@@ -85,7 +88,7 @@ __global__ void __launch_bounds__(PT_MK_THREADS) megakernel(const __grid_constan
         h.materialID = R(0);
         h.lightID = R(-1);
         int objectID = -1;
-        intersect_all<FEAT>(S, ps.org, shadow ? ps.shDir : ps.dir, h, objectID, shadow, ps.shObj, sign);
+        intersect_all<FEAT>(S, sphS, ps.org, shadow ? ps.shDir : ps.dir, h, objectID, shadow, ps.shObj, sign);
         if (!shadow) sign.set = 0u;  // shading moves the origin
         const StepResult r =
             shadow ? shade_shadow<TRACE>(ps, S, objectID, depth) : shade_primary<TRACE>(ps, S, h, objectID, depth);

@@ -37,14 +37,14 @@ template <typename R> PT_DI R cmf_lobe(R x, R mu, R s1, R s2) {
     return m_exp(-PT_LIT(R, 0.5) * t * t);
 }
 // The fit itself at wavelength `wave` (nm), for PT_EXT_ANALYTIC_CMF.
-template <typename R> PT_DI V3<R> cmf_analytic(R wave) {
+template <typename R> PT_CALL V3<R> cmf_analytic(R wave) {
     const R x = (PT_LIT(R, 1.056) * cmf_lobe(wave, PT_LIT(R, 599.8), PT_LIT(R, 37.9), PT_LIT(R, 31.0)) + PT_LIT(R, 0.362) * cmf_lobe(wave, PT_LIT(R, 442.0), PT_LIT(R, 16.0), PT_LIT(R, 26.7))) -
                     PT_LIT(R, 0.065) * cmf_lobe(wave, PT_LIT(R, 501.1), PT_LIT(R, 20.4), PT_LIT(R, 26.2));
     const R y = PT_LIT(R, 0.821) * cmf_lobe(wave, PT_LIT(R, 568.8), PT_LIT(R, 46.9), PT_LIT(R, 40.5)) + PT_LIT(R, 0.286) * cmf_lobe(wave, PT_LIT(R, 530.9), PT_LIT(R, 16.3), PT_LIT(R, 31.1));
     const R z = PT_LIT(R, 1.217) * cmf_lobe(wave, PT_LIT(R, 437.0), PT_LIT(R, 11.8), PT_LIT(R, 36.0)) + PT_LIT(R, 0.681) * cmf_lobe(wave, PT_LIT(R, 459.0), PT_LIT(R, 26.0), PT_LIT(R, 13.8));
     return v3<R>(x, y, z);
 }
-template <typename R> PT_DI V3<R> wave_to_xyz(const float* __restrict__ cie, R wave) {
+template <typename R> PT_CALL V3<R> wave_to_xyz(const float* __restrict__ cie, R wave) {
     V3<R> r = v3<R>(PT_LIT(R, 0.0), PT_LIT(R, 0.0), PT_LIT(R, 0.0));
     if ((wave >= PT_LIT(R, 360.0)) && (wave <= PT_LIT(R, 800.0))) {
         const int i3 = 3 * (int)(m_floor(wave) - PT_LIT(R, 360.0));
@@ -72,7 +72,7 @@ template <typename V, typename R = SOf<V>> PT_DI V evaluate_brdf(V l, ND<R> peak
 template <typename R> PT_DI R blackbody(R l, R T) {
     return (PT_LIT(R, 1.1910429724e-16) * (PT_LIT(R, 1.0) / pow_pos_int<5>(l))) / (m_exp(PT_LIT(R, 0.014387768775) / (l * T)) - PT_LIT(R, 1.0));
 }
-template <typename V, typename R = SOf<V>> PT_DI V emit(V l, ND<R> temperature_in, ND<R> luminosity) {
+template <typename V, typename R = SOf<V>> PT_CALL V emit(V l, ND<R> temperature_in, ND<R> luminosity) {
     const R T = m_fmax(temperature_in, PT_LIT(R, 0.0));
     const V4<R> lm = l * PT_LIT(R, 1e-9);
     const R peak = PT_LIT(R, 4.0956746759e-6) * pow_pos_int<5>(T);  // T >= 0
@@ -82,7 +82,7 @@ template <typename V, typename R = SOf<V>> PT_DI V emit(V l, ND<R> temperature_i
 }
 
 // RefractiveIndexBK7Glass, SC:1064-1073.
-template <typename R> PT_DI R bk7_index(R l) {
+template <typename R> PT_CALL R bk7_index(R l) {
     l *= PT_LIT(R, 1e-3);
     const R l2 = l * l;
     R n2 = PT_LIT(R, 1.0);
@@ -329,7 +329,7 @@ template <typename R> PT_DI const pt_material_ext* ext_material(const KScene& S,
     return (m->type == PT_BSDF_REFERENCE) ? nullptr : m;
 }
 // Refractive index of an extension dielectric at wavelength l (nm).
-template <typename R> PT_DI R ext_ior(const pt_material_ext& m, R l) {
+template <typename R> PT_CALL R ext_ior(const pt_material_ext& m, R l) {
     const R u = l * PT_LIT(R, 1e-3);
     const R u2 = u * u;
     if (m.type == PT_BSDF_CAUCHY) return m.p[0] + m.p[1] / u2;
@@ -340,22 +340,18 @@ template <typename R> PT_DI R ext_ior(const pt_material_ext& m, R l) {
     return m_sqrt(n2);
 }
 // Unpolarised Fresnel reflectance for relative index eta = n1 / n2 at
-// incidence cosine cosi (>= 0); 1 under total internal reflection.  *cost
-// receives the transmitted cosine.
-template <typename R> PT_DI R fresnel_dielectric(R eta, R cosi, R* cost) {
+// incidence cosine cosi (>= 0); 1 under total internal reflection (x), and
+// the transmitted cosine (y).
+template <typename R> PT_CALL V2<R> fresnel_dielectric(R eta, R cosi) {
     const R sin2t = (eta * eta) * (PT_LIT(R, 1.0) - cosi * cosi);
-    if (sin2t >= PT_LIT(R, 1.0)) {
-        *cost = PT_LIT(R, 0.0);
-        return PT_LIT(R, 1.0);
-    }
+    if (sin2t >= PT_LIT(R, 1.0)) return v2<R>(PT_LIT(R, 1.0), PT_LIT(R, 0.0));
     const R ct = m_sqrt(PT_LIT(R, 1.0) - sin2t);
     const R rs = (eta * cosi - ct) / (eta * cosi + ct);
     const R rp = (cosi - eta * ct) / (cosi + eta * ct);
-    *cost = ct;
-    return PT_LIT(R, 0.5) * (rs * rs + rp * rp);
+    return v2<R>(PT_LIT(R, 0.5) * (rs * rs + rp * rp), ct);
 }
 // The reflectance of a Lambertian extension material at the four wavelengths, / PI.
-template <typename V, typename R = SOf<V>> PT_DI V ext_lambert(const pt_material_ext& m, V l) {
+template <typename V, typename R = SOf<V>> PT_CALL V ext_lambert(const pt_material_ext& m, V l) {
     if (m.type == PT_BSDF_FLAT) return v4s<R>(m.p[0]) / PT_PI_R(R);
     const V4<R> x = v4<R>((l.x - m.p[2]) / m.p[3], (l.y - m.p[2]) / m.p[3], (l.z - m.p[2]) / m.p[3],
                         (l.w - m.p[2]) / m.p[3]);
@@ -397,15 +393,14 @@ PT_DI StepResult shade_specular(PathStateT<R>& ps, const pt_material_ext& m, con
     const bool inside = (ps.medium & 1) != 0;
     const R nh = ext_ior(m, ps.l.x);
     const R eta = inside ? nh : PT_LIT(R, 1.0) / nh;
-    R cost = PT_LIT(R, 0.0);
-    const R F = fresnel_dielectric(eta, cosi, &cost);
+    const V2<R> fr = fresnel_dielectric(eta, cosi);
+    const R F = fr.x, cost = fr.y;
     if (rnd<R>(ps.seed) < F) {
         ps.dir = ps.dir + n * (PT_LIT(R, 2.0) * cosi);
-        R ct;
         const R ny = ext_ior(m, ps.l.y), nz = ext_ior(m, ps.l.z), nw = ext_ior(m, ps.l.w);
-        const R Fy = fresnel_dielectric(inside ? ny : PT_LIT(R, 1.0) / ny, cosi, &ct);
-        const R Fz = fresnel_dielectric(inside ? nz : PT_LIT(R, 1.0) / nz, cosi, &ct);
-        const R Fw = fresnel_dielectric(inside ? nw : PT_LIT(R, 1.0) / nw, cosi, &ct);
+        const R Fy = fresnel_dielectric(inside ? ny : PT_LIT(R, 1.0) / ny, cosi).x;
+        const R Fz = fresnel_dielectric(inside ? nz : PT_LIT(R, 1.0) / nz, cosi).x;
+        const R Fw = fresnel_dielectric(inside ? nw : PT_LIT(R, 1.0) / nw, cosi).x;
         ps.rr = v4<R>(ps.rr.x, ps.rr.y * (Fy / F), ps.rr.z * (Fz / F), ps.rr.w * (Fw / F));
         if (TRACE) ps.ev |= PT_EV_SPECULAR;
     } else {

@@ -19,6 +19,9 @@
 // Largest object count the 1024-float object array can hold (planes, 5 floats).
 #define PT_MAX_SCENE_OBJECTS (PT_MAX_OBJECTS_SIZE / 5)
 
+// Largest sphere count (6 floats each).
+#define PT_MAX_SCENE_SPHERES (PT_MAX_OBJECTS_SIZE / 6)
+
 struct pt_scene_meta {
     int n[7];           // numObjects as integers (validated integral on upload)
     int offset[5];      // float offset of each primitive class in objects[]
@@ -39,7 +42,34 @@ struct KScene {
     pt_sdf_plugin plug[PT_MAX_LIVE_SDFS];
     float rot[PT_MAX_SCENE_OBJECTS][9];
     pt_scene_ext ext;  // full-form extensions; all zero: the reference's method
+    // Derived from the spheres on the host (pt_derive_cull): x, y, z and
+    // |pos|^2 - r^2 less the margin of the cull test, and a bound on |pos|.
+    float4 cull[PT_MAX_SCENE_SPHERES];
+    float cull_pmax;
 };
+
+// The cull test's margin, relative to |org|^2 + |pos|^2 + r^2: 2^-16 = 256
+// float roundings.  The test's own rounding errors and those of the exact
+// test (sphere_hit) add up to less than 100 (intersect_spheres).
+#define PT_CULL_EPS 1.52587890625e-05
+
+#if !defined(__CUDACC_RTC__)
+#include <cmath>
+// Fills the derived fields of a scene whose object arrays and counts are set.
+inline void pt_derive_cull(KScene* S) {
+    double pmax = 0.0;
+    for (int i = 0; i < S->meta.n[0] && i < PT_MAX_SCENE_SPHERES; i++) {
+        const float* o = S->objects + 6 * i;
+        const double x = o[0], y = o[1], z = o[2], r = o[3];
+        const double pp = x * x + y * y + z * z, rr = r * r;
+        // rounded down: a smaller value culls less
+        const float k = std::nextafter((float)(pp - rr - PT_CULL_EPS * (pp + rr)), -HUGE_VALF);
+        S->cull[i] = make_float4(o[0], o[1], o[2], k);
+        pmax = std::fmax(pmax, std::sqrt(pp));
+    }
+    S->cull_pmax = std::nextafter((float)pmax, HUGE_VALF);
+}
+#endif
 
 // Camera quantities that depend only on the push constants (SC:1456,
 // SC:1409-1418): derived once per block (megakernel) or per job (wavefront).

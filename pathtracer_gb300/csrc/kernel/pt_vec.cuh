@@ -24,6 +24,16 @@
 #include "../../../include/pt_mathf.h"
 
 #define PT_DI __device__ __forceinline__
+// One copy per kernel, called: for code that several places of the path loop
+// run or that few paths reach.  The path kernels are bound by instruction
+// fetch (no_instruction was their leading stall, 5 of 13 cycles an issue):
+// straight-line code runs at 0.95 issues a cycle and scheduler up to 32 KB
+// and at 0.3 to 0.5 beyond (measured on GB300 with unrolled loops of 4 to
+// 192 KB), and the smallest of them held 99 KB.  With emission, the CIE fit
+// and table, glass and the two lens faces in one copy each it holds 77 KB:
+// sphere scene 1024x1024x16 on the megakernel 8.6 -> 7.5 ms, batch of 16
+// sphere jobs 60.2 -> 53.6 ms, Cornell box staged 1.68 -> 1.61 ms.
+#define PT_CALL static __device__ __noinline__
 
 PT_DI float3 f3(float x, float y, float z) { return make_float3(x, y, z); }
 PT_DI float4 f4(float x, float y, float z, float w) { return make_float4(x, y, z, w); }

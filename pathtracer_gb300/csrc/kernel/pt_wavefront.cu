@@ -154,7 +154,7 @@ PT_DI bool route_ray(const WfArgs& A, const PoolView& v, const KScene& S, uint32
     h.materialID = 0.0f;
     h.lightID = -1.0f;
     int objectID = -1;
-    intersect_analytic(S, org, dir, h, objectID);
+    intersect_analytic(S, S.objects, org, dir, h, objectID, shadow);
     bool march = false;
     uint32_t set1 = 0;
     if (S.meta.n[5] > 0 && !(shadow && !shadow_needs_march(objectID, shObj))) {
@@ -470,6 +470,12 @@ __global__ void wf_persist_setup(const __grid_constant__ WfArgs A, uint64_t budg
 template <int FEAT, bool ONE>
 PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
     WfCounters& C = *A.counters;
+    // the launch's spheres, where lanes can read different ones at once
+    __shared__ float sphS[ONE ? 6 * PT_MAX_SCENE_SPHERES : 1];
+    if constexpr (ONE) {
+        for (int i = threadIdx.x; i < 6 * S1->meta.n[0]; i += kPersistThreads) sphS[i] = S1->objects[i];
+        __syncthreads();
+    }
     const uint64_t end = C.pk_end;
     const uint32_t job_lo = C.job_lo, job_hi = C.job_hi;
     const int lane = (int)(threadIdx.x & 31);
@@ -544,7 +550,7 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
             h.materialID = 0.0f;
             h.lightID = -1.0f;
             int objectID = -1;
-            intersect_all<FEAT>(S, ps.org, shadow ? ps.shDir : ps.dir, h, objectID, shadow, ps.shObj, sign);
+            intersect_all<FEAT>(S, ONE ? sphS : S.objects, ps.org, shadow ? ps.shDir : ps.dir, h, objectID, shadow, ps.shObj, sign);
             if (!shadow) sign.set = 0u;  // shading moves the origin
             const StepResult r = shadow ? shade_shadow<false>(ps, S, objectID, depth)
                                         : shade_primary<false>(ps, S, h, objectID, depth);

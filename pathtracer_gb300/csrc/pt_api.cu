@@ -274,6 +274,7 @@ int pt_upload_scene_ext(pt_ctx* ctx, const pt_ubo* ubo, const pt_scene_ext* ext)
         std::memset(&S.ext, 0, sizeof(S.ext));
     }
     refresh_plugins(ctx);
+    pt_derive_cull(&S);
 
     PT_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_cie, ubo->CIEXYZ1931, sizeof(float) * PT_CIE_TABLE_SIZE,
                                      cudaMemcpyHostToDevice, ctx->stream));

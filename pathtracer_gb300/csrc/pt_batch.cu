@@ -500,6 +500,7 @@ int add_scene(pt_batch* b, const pt_ubo* ubo, const pt_sdf_plugin* plugins, int 
     if (nplugins > 0) std::memcpy(S->plug, plugins, sizeof(pt_sdf_plugin) * (size_t)nplugins);
     S->meta.nplug = nplugins;
     S->meta.custom_base = custom_base;
+    pt_derive_cull(S);
     BatchScene bs;
     cudaError_t e = cudaMalloc(&bs.d_scene, sizeof(KScene));
     if (e == cudaSuccess) e = cudaMalloc(&bs.d_cie, sizeof(float) * PT_CIE_TABLE_SIZE);

@@ -112,6 +112,7 @@ int build_scene(const pt_ubo* ubo, const pt_sdf_plugin* plugins, int nplug, KSce
     S->meta.total_objects = n[0] + n[1] + n[2] + n[3] + n[4];
     if (nplug > 0) std::memcpy(S->plug, plugins, sizeof(pt_sdf_plugin) * (size_t)nplug);
     S->meta.nplug = nplug;
+    pt_derive_cull(S);
     return PT_OK;
 }
 
