@@ -194,19 +194,17 @@ template <typename R> struct LensGeomT {
 };
 using LensGeom = LensGeomT<float>;
 
-// SphereSliceIntersection, SC:366-417.
+// SphereSliceIntersection, SC:366-417, for a ray in the lens' frame.
 template <typename R>
-PT_DI bool slice_intersect(V3<R> org_w, V3<R> dir_w, const LensGeomT<R>& L, ND<R> sliceRadius, ND<R> sliceSize,
+PT_DI bool slice_intersect(V3<R> org, V3<R> dir, const LensGeomT<R>& L, ND<R> sliceRadius, ND<R> sliceSize,
                            bool is1st, ND<R> localSlicePos, bool isSideInvert, ND<R> mat, ND<R> light, HitT<R>& h,
                            int& isOutside) {
     const R sliceOffset = sliceRadius - sliceSize;
-    V3<R> org = mul_vm(org_w - L.pos, L.rot);
     if (is1st) {
         org.x += localSlicePos - sliceSize - sliceOffset;
     } else {
         org.x -= localSlicePos - sliceSize - sliceOffset;
     }
-    const V3<R> dir = mul_vm(dir_w, L.rot);
     const R b = R(2) * dot3(dir, org);
     const R c = dot3(org, org) - (sliceRadius * sliceRadius);
     const R disc = b * b - R(4) * c;
@@ -248,10 +246,11 @@ PT_DI bool lens_intersect(V3<R> org, V3<R> dir, const LensGeomT<R>& L, ND<R> mat
     R lensSlicePos = R(0.5) * (L.converging ? L.thickness : -L.thickness);
     if (L.converging) lensSlicePos += lensThicknessHalf;
     const R sliceRadius = R(2) * L.focal;
+    const V3<R> org_l = mul_vm(org - L.pos, L.rot), dir_l = mul_vm(dir, L.rot);
     bool hit = false;
 #pragma unroll 1
     for (int i = 0; i < 2; i++) {
-        if (slice_intersect(org, dir, L, sliceRadius, lensThicknessHalf, i == 0, lensSlicePos, !L.converging, mat,
+        if (slice_intersect(org_l, dir_l, L, sliceRadius, lensThicknessHalf, i == 0, lensSlicePos, !L.converging, mat,
                             light, h, isOutside))
             hit = true;
     }
@@ -653,6 +652,11 @@ PT_DI R plugin_sdf(int kind, int slot, V p) {
         default: return R(PT_MAXDIST);
     }
 }
+// One out-of-line copy, for the places that seldom evaluate an SDF.
+template <uint32_t KINDS, typename V, typename R = SOf<V>>
+static __device__ __noinline__ R plugin_sdf_cold(int kind, int slot, V p) {
+    return plugin_sdf<KINDS>(kind, slot, p);
+}
 template <typename V, typename R = SOf<V>> PT_DI R plugin_material(const pt_sdf_plugin& pl, int slot, V p) {
     if (pl.material_mode == PT_SDFMAT_CONSTANT) return R(pl.material[0]);
     switch (pl.kind) {
@@ -709,13 +713,16 @@ template <typename V, typename R = SOf<V>> PT_DI R scene_sdf(const KScene& S, V 
 // the SDFs they share in the same trip: over each lane's own set, lanes with
 // {0, 1} and lanes with {1} ran SDF 1 in different trips (10.5 of 32 lanes
 // per instruction on menger + terrain).
-template <uint32_t KINDS = PT_SDF_KINDS, typename V, typename R = SOf<V>>
+// COLD: by calls of the plug-ins' one out-of-line copy (plugin_sdf_cold).
+template <uint32_t KINDS = PT_SDF_KINDS, bool COLD = false, typename V, typename R = SOf<V>>
 PT_DI R scene_sdf_sel(const KScene& S, V p, uint32_t set1, uint32_t walk, int& sel) {
     R sdf = R(PT_MAXDIST);
     sel = -1;
 #if defined(PT_ONE_SDF)
     if (set1 & 1u) {  // as in scene_sdf
-        const R di = plugin_sdf<KINDS>(PT_SDF_CUSTOM, S.meta.custom_base, p - sdf_pos<R>(S, 0));
+        const V3<R> q = p - sdf_pos<R>(S, 0);
+        const R di = COLD ? plugin_sdf_cold<KINDS>(PT_SDF_CUSTOM, S.meta.custom_base, q)
+                          : plugin_sdf<KINDS>(PT_SDF_CUSTOM, S.meta.custom_base, q);
         if (!(sdf < di)) sel = 0;
         sdf = m_fmin(sdf, di);
     }
@@ -728,7 +735,9 @@ PT_DI R scene_sdf_sel(const KScene& S, V p, uint32_t set1, uint32_t walk, int& s
         if (!((bits >> i) & 1u)) continue;
         const int kind = S.plug[i].kind;
         if (kind != PT_SDF_NONE) {
-            const R di = plugin_sdf<KINDS>(kind, S.meta.custom_base + i, p - sdf_pos<R>(S, i));
+            const V3<R> q = p - sdf_pos<R>(S, i);
+            const R di = COLD ? plugin_sdf_cold<KINDS>(kind, S.meta.custom_base + i, q)
+                              : plugin_sdf<KINDS>(kind, S.meta.custom_base + i, q);
             if (!(sdf < di)) sel = i;
             sdf = m_fmin(sdf, di);
         }
@@ -754,7 +763,7 @@ static __device__ __noinline__ R scene_sdf_material(const KScene& S, V p, uint32
         const pt_sdf_plugin pl = S.plug[i];
         if (pl.kind != PT_SDF_NONE) {
             const V3<R> q = p - sdf_pos<R>(S, i);
-            const R di = plugin_sdf(pl.kind, S.meta.custom_base + i, q);
+            const R di = plugin_sdf_cold<PT_SDF_KINDS>(pl.kind, S.meta.custom_base + i, q);
             mat = (sdf < di) ? mat : plugin_material(pl, S.meta.custom_base + i, q);
             sdf = m_fmin(sdf, di);
         }

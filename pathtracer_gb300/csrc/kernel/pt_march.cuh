@@ -5,7 +5,7 @@
 // the same source.
 #pragma once
 
-#include "pt_path.cuh"
+#include "pt_geometry.cuh"
 #include "pt_wavefront.h"
 
 #if defined(PT_JIT_USER_SDF)
@@ -214,18 +214,17 @@ template <typename P> PT_DI float3 probe_point(const P& p, int j) {
     return (j & 1) ? f3(p.x - mx, p.y - my, p.z - mz) : f3(p.x + ex, p.y + ey, p.z + ez);
 }
 
-// The normal stage's evaluation: out of line in run-time compiled kernels,
-// where a second inlined copy of a long snippet cost registers and
-// instruction cache (12-iteration mandelbulb 131.3 against 130.0 ms); inlined
-// it is as fast or faster for the shipped plug-ins.
-#if defined(PT_JIT_USER_SDF)
-template <uint32_t KINDS>
-static __device__ __noinline__ float probe_sdf(const KScene& S, float3 q, uint32_t set1, uint32_t walk) {
-#else
+// The normal stage's evaluation: in run-time compiled kernels by calls of the
+// plug-ins' cold copy, since a second inlined copy of a long snippet cost
+// registers and instruction cache (12-iteration mandelbulb 131.3 against
+// 130.0 ms); inlined it is as fast or faster for the shipped plug-ins.
 template <uint32_t KINDS> PT_DI float probe_sdf(const KScene& S, float3 q, uint32_t set1, uint32_t walk) {
-#endif
     int sel;
+#if defined(PT_JIT_USER_SDF)
+    return scene_sdf_sel<KINDS, true>(S, q, set1, walk, sel);
+#else
     return scene_sdf_sel<KINDS>(S, q, set1, walk, sel);
+#endif
 }
 
 // Normals and materials of records [from, from + n), n <= kNormalBatch, into
@@ -539,7 +538,9 @@ PT_DI void march_rays(const WfArgs& A) {
 // host picks the smallest that covers a dispatch.  Code of kinds that a
 // scene does not have cost menger + terrain 10 % and the shipped mandelbulb
 // 2 % (instruction cache, registers).
-#if defined(PT_JIT_USER_SDF)
+#if defined(PT_NO_MARCH_KERNELS)
+// (a translation unit that takes only the helpers)
+#elif defined(PT_JIT_USER_SDF)
 __global__ void PT_MARCH_BOUNDS wf_march(const __grid_constant__ WfArgs A) { march_rays<true, PT_SDF_KINDS>(A); }
 #else
 constexpr uint32_t kKindsBulb = 1u << PT_SDF_MANDELBULB;
