@@ -29,6 +29,8 @@ CUDA_SOURCES = [
     "kernel/pt_fp64.cu",
     "kernel/pt_wavefront.cu",
     "kernel/pt_wavefront_checked.cu",
+    "kernel/pt_persist.cu",
+    "kernel/pt_persist_checked.cu",
     "pt_api.cu",
     "pt_engine.cu",
     "pt_noalloc.cu",

@@ -1,8 +1,9 @@
 // pt_megakernel_analytic.cu — the plain megakernel's variants for scenes
 // without SDFs (pt_megakernel_body.cuh).  Their shading calls the larger
-// pt_mathf functions out of line: the loop stays small enough for the
-// instruction cache, which these compute-bound variants measurably need.
+// pt_mathf functions, quotients and roots out of line: these variants are
+// bound by instruction fetch (PT_CALL in pt_vec.cuh).
 #define PTM_OUTLINE
+#define PT_COMPACT
 #include <cuda_runtime.h>
 
 #include "pt_megakernel_body.cuh"

@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(PT_MK_THREADS) megakernel(const __grid_constan
         intersect_all<FEAT>(S, sphS, ps.org, shadow ? ps.shDir : ps.dir, h, objectID, shadow, ps.shObj, sign);
         if (!shadow) sign.set = 0u;  // shading moves the origin
         const StepResult r =
-            shadow ? shade_shadow<TRACE>(ps, S, objectID, depth) : shade_primary<TRACE>(ps, S, h, objectID, depth);
+            shadow ? shade_shadow<TRACE>(ps, S, objectID, depth) : shade_primary<TRACE, FEAT>(ps, S, h, objectID, depth);
         shadow = (r == STEP_SHADOW);
         if (TRACE && r != STEP_SHADOW) {
             const size_t p = pix * (size_t)spf + (size_t)(k - 1);

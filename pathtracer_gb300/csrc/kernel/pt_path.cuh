@@ -59,7 +59,7 @@ template <typename R> PT_CALL V3<R> wave_to_xyz(const float* __restrict__ cie, R
 // SpectralPowerDistribution / EvaluateBRDF, SC:1030-1038, SC:1075-1080.
 template <typename V, typename R = SOf<V>> PT_DI V evaluate_brdf(V l, ND<R> peak, ND<R> sigma, ND<R> invertf) {
     const R den = PT_LIT(R, 2.0) * sigma * sigma;
-    const V4<R> x = v4<R>((l.x - peak) / den, (l.y - peak) / den, (l.z - peak) / den, (l.w - peak) / den);
+    const V4<R> x = v4<R>(l.x - peak, l.y - peak, l.z - peak, l.w - peak) / den;
     const V4<R> r = v4<R>(m_exp(-x.x * x.x), m_exp(-x.y * x.y), m_exp(-x.z * x.z), m_exp(-x.w * x.w));
     const R a = (R)(int)invertf;
     const V4<R> s = v4<R>(mix_glsl(r.x, PT_LIT(R, 1.0) - r.x, a), mix_glsl(r.y, PT_LIT(R, 1.0) - r.y, a), mix_glsl(r.z, PT_LIT(R, 1.0) - r.z, a),
@@ -69,15 +69,15 @@ template <typename V, typename R = SOf<V>> PT_DI V evaluate_brdf(V l, ND<R> peak
 
 // BlackBodyRadiation / Emit, SC:1040-1055.
 // pow(l, -5) as ptm_powf computes it, 1 / l^5 by binary powering (l > 0).
-template <typename R> PT_DI R blackbody(R l, R T) {
-    return (PT_LIT(R, 1.1910429724e-16) * (PT_LIT(R, 1.0) / pow_pos_int<5>(l))) / (m_exp(PT_LIT(R, 0.014387768775) / (l * T)) - PT_LIT(R, 1.0));
-}
 template <typename V, typename R = SOf<V>> PT_CALL V emit(V l, ND<R> temperature_in, ND<R> luminosity) {
     const R T = m_fmax(temperature_in, PT_LIT(R, 0.0));
     const V4<R> lm = l * PT_LIT(R, 1e-9);
     const R peak = PT_LIT(R, 4.0956746759e-6) * pow_pos_int<5>(T);  // T >= 0
-    const V4<R> e = v4<R>(blackbody(lm.x, T) / peak, blackbody(lm.y, T) / peak, blackbody(lm.z, T) / peak,
-                        blackbody(lm.w, T) / peak);
+    const V4<R> one = v4s<R>(PT_LIT(R, 1.0));
+    const V4<R> l5 = m_div4(one, v4<R>(pow_pos_int<5>(lm.x), pow_pos_int<5>(lm.y), pow_pos_int<5>(lm.z), pow_pos_int<5>(lm.w)));
+    const V4<R> x = m_div4(v4s<R>(PT_LIT(R, 0.014387768775)), lm * T);
+    const V4<R> ex = v4<R>(m_exp(x.x) - PT_LIT(R, 1.0), m_exp(x.y) - PT_LIT(R, 1.0), m_exp(x.z) - PT_LIT(R, 1.0), m_exp(x.w) - PT_LIT(R, 1.0));
+    const V4<R> e = m_div4(l5 * PT_LIT(R, 1.1910429724e-16), ex) / peak;
     return e * m_fmax(luminosity, PT_LIT(R, 0.0));
 }
 
@@ -97,7 +97,7 @@ template <typename V, typename R = SOf<V>> PT_DI V to_world(V v, V n) {
     V3<R> b1 = v3<R>(PT_LIT(R, 0.0), -PT_LIT(R, 1.0), PT_LIT(R, 0.0));
     V3<R> b2 = v3<R>(-PT_LIT(R, 1.0), PT_LIT(R, 0.0), PT_LIT(R, 0.0));
     if (n.z >= -PT_LIT(R, 0.9999999)) {
-        const R a = PT_LIT(R, 1.0) / (PT_LIT(R, 1.0) + n.z);
+        const R a = m_div(PT_LIT(R, 1.0), PT_LIT(R, 1.0) + n.z);
         const R b = -n.x * n.y * a;
         b1 = v3<R>(PT_LIT(R, 1.0) - (n.x * n.x * a), b, -n.x);
         b2 = v3<R>(b, PT_LIT(R, 1.0) - (n.y * n.y * a), -n.y);
@@ -123,7 +123,11 @@ template <typename R> PT_DI V2<R> light_mix(const KScene& S, R lightID) {
 // SampleRandomLightSource, SC:1225-1285, quirks included: the lens branch
 // compares with the box count (SC:1264) and the cyclide branch with the lens
 // count (SC:1275).  Object reads are guarded: these indices come from data.
-template <typename R>
+// FEAT: the scene's primitive classes; without boxes, lenses and cyclides no
+// index reaches their branches (5 KB of the sphere megakernel, 7.3 -> 6.4 ms
+// on 1024x1024x16; the persistent kernel keeps them: it measured 5 % slower
+// without, by its code's layout).
+template <int FEAT, typename R>
 PT_DI int sample_random_light(const KScene& S, uint32_t& seed, R& boundingRadius, V3<R>& pos, R& lightID,
                               int& pick) {
     const int randomLight = (int)m_floor(rnd<R>(seed) * S.numObjects[6]);
@@ -148,33 +152,35 @@ PT_DI int sample_random_light(const KScene& S, uint32_t& seed, R& boundingRadius
         lightID = (R)((int)s_obj(S, b + 4) - 1);
         return result;
     }
-    L -= n[1];
-    offset += 5 * n[1];
-    if (L < n[2]) {
-        const int b = 11 * L + offset;
-        boundingRadius = PT_LIT(R, 0.5) * length3(v3<R>(s_obj(S, b + 6), s_obj(S, b + 7), s_obj(S, b + 8)));
-        pos = v3<R>(s_obj(S, b), s_obj(S, b + 1), s_obj(S, b + 2));
-        lightID = (R)((int)s_obj(S, b + 10) - 1);
-        return result;
-    }
-    L -= n[2];
-    offset += 11 * n[2];
-    if (L < n[2]) {
-        const int b = 12 * L + offset;
-        const R r = s_obj(S, b + 6), th = s_obj(S, b + 8);
-        boundingRadius = m_sqrt((r * r) + (PT_LIT(R, 0.25) * th * th));
-        pos = v3<R>(s_obj(S, b), s_obj(S, b + 1), s_obj(S, b + 2));
-        lightID = (R)((int)s_obj(S, b + 11) - 1);
-        return result;
-    }
-    L -= n[3];
-    offset += 12 * n[3];
-    if (L < n[3]) {
-        const int b = 16 * L + offset;
-        boundingRadius = m_sqrt(s_obj(S, b + 13));
-        pos = v3<R>(s_obj(S, b), s_obj(S, b + 1), s_obj(S, b + 2));
-        lightID = (R)((int)s_obj(S, b + 15) - 1);
-        return result;
+    if constexpr ((FEAT & PT_FEAT_ANALYTIC) != 0) {
+        L -= n[1];
+        offset += 5 * n[1];
+        if (L < n[2]) {
+            const int b = 11 * L + offset;
+            boundingRadius = PT_LIT(R, 0.5) * length3(v3<R>(s_obj(S, b + 6), s_obj(S, b + 7), s_obj(S, b + 8)));
+            pos = v3<R>(s_obj(S, b), s_obj(S, b + 1), s_obj(S, b + 2));
+            lightID = (R)((int)s_obj(S, b + 10) - 1);
+            return result;
+        }
+        L -= n[2];
+        offset += 11 * n[2];
+        if (L < n[2]) {
+            const int b = 12 * L + offset;
+            const R r = s_obj(S, b + 6), th = s_obj(S, b + 8);
+            boundingRadius = m_sqrt((r * r) + (PT_LIT(R, 0.25) * th * th));
+            pos = v3<R>(s_obj(S, b), s_obj(S, b + 1), s_obj(S, b + 2));
+            lightID = (R)((int)s_obj(S, b + 11) - 1);
+            return result;
+        }
+        L -= n[3];
+        offset += 12 * n[3];
+        if (L < n[3]) {
+            const int b = 16 * L + offset;
+            boundingRadius = m_sqrt(s_obj(S, b + 13));
+            pos = v3<R>(s_obj(S, b), s_obj(S, b + 1), s_obj(S, b + 2));
+            lightID = (R)((int)s_obj(S, b + 15) - 1);
+            return result;
+        }
     }
     return 0;
 }
@@ -218,8 +224,8 @@ PT_DI void start_sample(PathStateT<R>& ps, const KScene& S, const pt_push& pc, c
     const R jx = PT_LIT(R, 2.0) * rnd<R>(seed) - PT_LIT(R, 0.5);
     const R jy = PT_LIT(R, 2.0) * rnd<R>(seed) - PT_LIT(R, 0.5);
     const R sc = -pc.cameraSize * PT_LIT(R, 0.5);
-    const R u = (uvx + jx / (R)W) * sc;
-    const R v = (uvy + jy / (R)H) * sc;
+    const R u = (uvx + m_div(jx, (R)W)) * sc;
+    const R v = (uvy + m_div(jy, (R)H)) * sc;
     const V3<R> camPos = v3<R>(pc.cameraPosX, pc.cameraPosY, pc.cameraPosZ);
     V3<R> org = camPos + mul_vm(v3<R>(u, v, PT_LIT(R, 0.0)), cam.cam);
     const R rx = rnd<R>(seed);
@@ -260,7 +266,7 @@ PT_DI void start_sample(PathStateT<R>& ps, const KScene& S, const pt_push& pc, c
                 n1 = bk7_index(lam);
                 n2 = PT_LIT(R, 1.0);
             }
-            const R n12 = n1 / n2;
+            const R n12 = m_div(n1, n2);
             lam = lam * n12;
             org = fma3s(dir, h.hitdist, org);
             dir = refract3(dir, h.normal, n12);
@@ -303,7 +309,7 @@ PT_DI StepResult roulette(PathStateT<R>& ps, int depth) {
         ps.bounce++;
         return STEP_TERMINATED;
     }
-    ps.rr = ps.rr * (PT_LIT(R, 1.0) / rp);
+    ps.rr = ps.rr * m_div(PT_LIT(R, 1.0), rp);
     ps.bounce++;
     return (ps.bounce >= depth) ? STEP_TERMINATED : STEP_CONTINUE;
 }
@@ -418,7 +424,7 @@ PT_DI StepResult shade_specular(PathStateT<R>& ps, const pt_material_ext& m, con
 
 // TraceRay after Intersection (SC:1345-1391) for the path ray: emitter, miss,
 // or BRDF sampling + SampleLightSource (SC:1298-1343) up to the shadow ray.
-template <bool TRACE, typename R>
+template <bool TRACE, int FEAT = PT_FEAT_ALL, typename R>
 PT_DI StepResult shade_primary(PathStateT<R>& ps, const KScene& S, const HitT<R>& h, int objectID, int depth) {
     if (TRACE) ps.ev = PT_EV_VALID;
     if (!(h.hitdist < R(PT_MAXDIST))) {
@@ -459,7 +465,7 @@ PT_DI StepResult shade_primary(PathStateT<R>& ps, const KScene& S, const HitT<R>
         m_sincos(phi, &sp, &cp);
         ps.dir = normalize3(ps.nrm + v3<R>(cp * cosTheta, sp * cosTheta, sinTheta));
     }
-    ps.brdfPdf = dot3(ps.dir, ps.nrm) / PT_PI_R(R);
+    ps.brdfPdf = m_div(dot3(ps.dir, ps.nrm), PT_PI_R(R));
     const R numLights = S.numObjects[6];
     int pick = 0;
     uint32_t shadowState = 0;
@@ -468,8 +474,9 @@ PT_DI StepResult shade_primary(PathStateT<R>& ps, const KScene& S, const HitT<R>
         R boundingRadius = PT_LIT(R, 0.0);
         V3<R> lightPos = v3<R>(PT_LIT(R, 0.0), PT_LIT(R, 0.0), PT_LIT(R, 0.0));
         ps.shLightID = -PT_LIT(R, 1.0);
-        ps.shObj = sample_random_light(S, ps.seed, boundingRadius, lightPos, ps.shLightID, pick);
-        const R invLightDistance = PT_LIT(R, 1.0) / length3(lightPos - ps.org);
+        ps.shObj = sample_random_light<FEAT>(S, ps.seed, boundingRadius, lightPos, ps.shLightID, pick);
+        const V3<R> toLight = lightPos - ps.org;
+        const R invLightDistance = m_invsqrt(dot3(toLight, toLight));
         const V3<R> lightDir = (lightPos - ps.org) * invLightDistance;
         const R sinthetaMax = m_fmin(boundingRadius * invLightDistance, PT_LIT(R, 1.0));
         const R costhetaMax = m_sqrt(PT_LIT(R, 1.0) - sinthetaMax * sinthetaMax);
@@ -484,9 +491,9 @@ PT_DI StepResult shade_primary(PathStateT<R>& ps, const KScene& S, const HitT<R>
             m_sincos(phi, &sp, &cp);
             ps.shDir = to_world(normalize3(v3<R>(cp * sinTheta, sp * sinTheta, cosTheta + PT_LIT(R, 1.0))), lightDir);
         }
-        ps.lightPdf = PT_LIT(R, 1.0) / numLights;
-        ps.lightPdf *= dot3(ps.shDir, lightDir) / (PT_PI_R(R) * (PT_LIT(R, 1.0) - costhetaMax * costhetaMax));
-        ps.mis = ps.brdfPdf * ps.brdfPdf / (ps.brdfPdf * ps.brdfPdf + ps.lightPdf * ps.lightPdf);
+        ps.lightPdf = m_div(PT_LIT(R, 1.0), numLights);
+        ps.lightPdf *= m_div(dot3(ps.shDir, lightDir), PT_PI_R(R) * (PT_LIT(R, 1.0) - costhetaMax * costhetaMax));
+        ps.mis = m_div(ps.brdfPdf * ps.brdfPdf, ps.brdfPdf * ps.brdfPdf + ps.lightPdf * ps.lightPdf);
         ps.cosL = dot3(ps.shDir, ps.nrm);
         const R deathProbability = PT_LIT(R, 1.25) * m_fmax(ps.mis - PT_LIT(R, 0.2), PT_LIT(R, 0.0));
         if (ps.cosL >= PT_LIT(R, 0.0)) {
@@ -498,7 +505,7 @@ PT_DI StepResult shade_primary(PathStateT<R>& ps, const KScene& S, const HitT<R>
             }
         }
     } else {
-        ps.mis = ps.brdfPdf * ps.brdfPdf / (ps.brdfPdf * ps.brdfPdf + PT_LIT(R, 0.0) * PT_LIT(R, 0.0));
+        ps.mis = m_div(ps.brdfPdf * ps.brdfPdf, ps.brdfPdf * ps.brdfPdf + PT_LIT(R, 0.0) * PT_LIT(R, 0.0));
     }
     if (TRACE) ps.ev |= ((uint32_t)(pick & 0x7F) << PT_EV_LIGHT_SHIFT) | (shadowState << PT_EV_SHADOW_SHIFT);
     if (shadow) return STEP_SHADOW;

@@ -34,6 +34,17 @@
 // sphere scene 1024x1024x16 on the megakernel 8.6 -> 7.5 ms, batch of 16
 // sphere jobs 60.2 -> 53.6 ms, Cornell box staged 1.68 -> 1.61 ms.
 #define PT_CALL static __device__ __noinline__
+// Quotients, roots and reciprocals of the path loop: calls in a translation
+// unit that defines PT_COMPACT (an inlined IEEE division takes 20
+// instructions, a square root 16), inlined elsewhere.  As calls: batch of 16
+// sphere jobs on the persistent kernel 34.8 -> 31.4 ms, sphere scene on the
+// megakernel 7.5 -> 7.3; the staged stages, which wait for memory, ran 1 to 3 %
+// slower with them.
+#if defined(PT_COMPACT)
+#define PT_QUOT PT_CALL
+#else
+#define PT_QUOT PT_DI
+#endif
 
 PT_DI float3 f3(float x, float y, float z) { return make_float3(x, y, z); }
 PT_DI float4 f4(float x, float y, float z, float w) { return make_float4(x, y, z, w); }
@@ -110,7 +121,13 @@ PT_DI float3 operator-(float3 a) { return f3(-a.x, -a.y, -a.z); }
 PT_DI float4 operator+(float4 a, float4 b) { return f4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 PT_DI float4 operator*(float4 a, float4 b) { return f4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
 PT_DI float4 operator*(float4 a, float s) { return f4(a.x * s, a.y * s, a.z * s, a.w * s); }
-PT_DI float4 operator/(float4 a, float s) { return f4(a.x / s, a.y / s, a.z / s, a.w / s); }
+PT_QUOT float m_div(float a, float b) { return a / b; }
+PT_DI double m_div(double a, double b) { return a / b; }
+PT_QUOT float4 m_div4(float4 a, float4 b) { return f4(a.x / b.x, a.y / b.y, a.z / b.z, a.w / b.w); }
+PT_QUOT float m_invsqrt(float x) { return 1.0f / sqrtf(x); }
+PT_DI double m_invsqrt(double x) { return 1.0 / sqrt(x); }
+PT_QUOT float4 m_div4s(float4 a, float s) { return f4(a.x / s, a.y / s, a.z / s, a.w / s); }
+PT_DI float4 operator/(float4 a, float s) { return m_div4s(a, s); }
 
 // The same operators for double vectors (the FP64 reference renderer).
 PT_DI double3 operator+(double3 a, double3 b) { return double3{a.x + b.x, a.y + b.y, a.z + b.z}; }
@@ -122,13 +139,13 @@ PT_DI double3 operator-(double3 a) { return double3{-a.x, -a.y, -a.z}; }
 PT_DI double4_16a operator+(double4_16a a, double4_16a b) { return double4_16a{a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w}; }
 PT_DI double4_16a operator*(double4_16a a, double4_16a b) { return double4_16a{a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w}; }
 PT_DI double4_16a operator*(double4_16a a, double s) { return double4_16a{a.x * s, a.y * s, a.z * s, a.w * s}; }
+PT_DI double4_16a m_div4(double4_16a a, double4_16a b) { return double4_16a{a.x / b.x, a.y / b.y, a.z / b.z, a.w / b.w}; }
 PT_DI double4_16a operator/(double4_16a a, double s) { return double4_16a{a.x / s, a.y / s, a.z / s, a.w / s}; }
 
 template <typename V> PT_DI auto dot3(V a, V b) -> decltype(a.x) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 template <typename V> PT_DI auto length3(V a) -> decltype(a.x) { return m_sqrt(dot3(a, a)); }
 template <typename V> PT_DI V normalize3(V a) {
-    const auto inv = decltype(a.x)(1) / m_sqrt(dot3(a, a));
-    return a * inv;
+    return a * m_invsqrt(dot3(a, a));
 }
 template <typename V> PT_DI V fma3(V a, V b, V c) {
     return V{m_fma(a.x, b.x, c.x), m_fma(a.y, b.y, c.y), m_fma(a.z, b.z, c.z)};

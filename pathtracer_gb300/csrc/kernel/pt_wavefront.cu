@@ -24,7 +24,7 @@
 // and applies Rendering/Accumulate — the same float operations, in the same
 // order, as the megakernel and the shader, so results are bit-identical.
 // The larger pt_mathf functions are called out of line here (smaller stage
-// and persistent kernels); the SDF plug-ins use inlined math regardless.
+// kernels); the SDF plug-ins use inlined math regardless.
 //
 // pt_wavefront_checked.cu compiles this file a second time with
 // PT_DEBUG_CHECKS (every queue, pool-slot, ring and sample index checked
@@ -39,18 +39,10 @@
 
 #include "pt_march.cuh"
 #include "pt_path.cuh"
+#include "pt_ring.cuh"
 #include "pt_wavefront.h"
 
 namespace {
-
-// The flags word of s8: bit 30 the shadow-ray flag (kShadowFlag), bits
-// 28-29 the extension dielectrics' path bits (PathState::medium), the bounce
-// count below.
-constexpr uint32_t kMediumShift = 28;
-constexpr uint32_t kBounceMask = (1u << kMediumShift) - 1u;
-PT_DI uint32_t bounce_word(const PathState& ps) {
-    return ((uint32_t)ps.medium << kMediumShift) | ((uint32_t)ps.bounce & kBounceMask);
-}
 
 // A shadow-ray result's state: the bounce's next ray (s0, s1), the NEE
 // term and the next throughput made with the shadow ray (s3, s5: see
@@ -107,34 +99,12 @@ PT_DI void store_new_sample(const PoolView& v, uint32_t slot, const PathState& p
     v.s8[slot] = make_uint4(ps.seed, bounce_word(ps), sample, job_word(job, ps.shObj));
 }
 
-// The ring entry of the pass that holds global sample s: the last pass in
-// [lo, hi) with first <= s (passes are appended in increasing order of first).
-PT_DI uint32_t find_job(const WfJob* __restrict__ jobs, uint32_t cap, uint32_t lo, uint32_t hi, uint64_t s) {
-    // invariant: jobs[lo % cap].first <= s < jobs[hi % cap].first (or hi is the end)
-    while (hi - lo > 1) {
-        const uint32_t mid = lo + ((hi - lo) >> 1);
-        if (jobs[mid % cap].first <= s) {
-            lo = mid;
-        } else {
-            hi = mid;
-        }
-    }
-    return lo % cap;
-}
-
 // Sample id s of a dispatch: k = s / (W*H), pixel = s % (W*H).  The colour
 // buffer is [k][pixel], so `resolve` reads it coalesced; traces use the
 // megakernel's path index pixel * spf + k.
 PT_DI size_t trace_index(const pt_push& pc, uint32_t s) {
     const uint32_t npix = (uint32_t)pc.resolution[0] * (uint32_t)pc.resolution[1];
     return (size_t)(s % npix) * (size_t)pc.samplesPerFrame + (size_t)(s / npix);
-}
-
-// Samples of every pass added so far: the end of the last pass.
-PT_DI uint64_t jobs_total(const WfArgs& A, uint32_t hi) {
-    if (hi == 0) return 0;
-    const WfJob& L = A.jobs[(hi - 1) % A.job_cap];
-    return L.first + (uint64_t)L.count;
 }
 
 // Intersection for a ray a stage has just produced (the reference's
@@ -238,16 +208,6 @@ __global__ void wf_job_add(const __grid_constant__ WfArgs A, const WfJob job, ui
     WfCounters& C = *A.counters;
     C.job_hi = index + 1;
     C.job_lo = lo;
-}
-
-// Adds 1 to jobs[job].finished for every lane with pred, one atomic per
-// distinct job in the warp.  Called by all 32 lanes.
-PT_DI void count_finished(WfJob* __restrict__ jobs, uint32_t job, bool pred) {
-    const unsigned active = __ballot_sync(0xffffffffu, pred);
-    if (!active) return;
-    const unsigned same = __match_any_sync(0xffffffffu, pred ? job : 0xffffffffu);
-    if (pred && (__ffs(same & active) - 1) == (int)(threadIdx.x & 31))
-        atomicAdd(&jobs[job].finished, (uint32_t)__popc(same & active));
 }
 
 // A primary hit reads neither the shadow-ray fields (s2, s3) nor the BRDF
@@ -441,143 +401,6 @@ __global__ void PT_SHADE_BOUNDS wf_shade(const __grid_constant__ WfArgs A) {
     }
 }
 
-// Persistent mode: the megakernel's per-thread path loop (one intersect_all
-// call site per iteration for primary and shadow rays alike) over the samples
-// of every pass in the ring.  A lane whose path ends takes the next sample
-// at once, from a chunk its warp claimed with one atomic, so lanes stay busy
-// across pixels, samples and passes; no path state leaves registers.  Each
-// sample's colour goes to its pass's colour buffer, which `resolve` sums in
-// sample order, so results equal the megakernel's bit for bit.  Suited to
-// scenes without SDFs, where lanes of a warp do similar work per ray; SDF
-// marching diverges per lane and belongs to the staged kernels above.
-constexpr uint32_t kPersistChunk = 256;
-
-__global__ void wf_persist_setup(const __grid_constant__ WfArgs A, uint64_t budget) {
-    WfCounters& C = *A.counters;
-    const uint64_t total = jobs_total(A, C.job_hi);
-    const uint64_t begin = C.pk_end;  // warps of the last launch may have claimed past it
-    const uint64_t end = (total - begin > budget) ? begin + budget : total;
-    C.next_sample = begin;
-    C.pk_end = end;
-    C.total = total;
-    C.iterations += 1;
-}
-
-// The persistent path loop.  ONE: every sample of the launch belongs to one
-// pass, whose scene S1 is the launch's parameter (the constant bank, as
-// for the megakernel); otherwise each lane reads its pass's scene through
-// the pass's pointer.
-template <int FEAT, bool ONE>
-PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
-    WfCounters& C = *A.counters;
-    // the launch's spheres, where lanes can read different ones at once
-    __shared__ float sphS[ONE ? 6 * PT_MAX_SCENE_SPHERES : 1];
-    if constexpr (ONE) {
-        for (int i = threadIdx.x; i < 6 * S1->meta.n[0]; i += kPersistThreads) sphS[i] = S1->objects[i];
-        __syncthreads();
-    }
-    const uint64_t end = C.pk_end;
-    const uint32_t job_lo = C.job_lo, job_hi = C.job_hi;
-    const int lane = (int)(threadIdx.x & 31);
-    const unsigned lt = (1u << lane) - 1u;
-    uint64_t cbase = 0;   // warp-uniform: unassigned samples of the warp's chunk
-    uint32_t cleft = 0;
-    uint32_t cjob = 0;      // warp-uniform: pass of the chunk's first sample,
-    uint64_t cjob_end = 0;  // and the end of its sample range
-    bool exhausted = false;  // warp-uniform: no sample left below `end`
-    bool active = false, shadow = false;
-    uint32_t job = 0, local = 0;
-    PathState ps;
-    OriginSignT<float> sign{0.0f, 0u};
-    for (;;) {
-        // Refill idle lanes from the warp's chunk, claiming chunks as needed,
-        // once persist_refill lanes are idle (or none is busy): new samples
-        // start together instead of one lane at a time.
-        unsigned need = __ballot_sync(0xffffffffu, !active);
-        if (__popc(need) < A.persist_refill && need != 0xffffffffu) need = 0u;
-        while (need && !exhausted) {
-            if (cleft == 0) {
-                unsigned long long b = 0;
-                if (lane == 0) b = atomicAdd(reinterpret_cast<unsigned long long*>(&C.next_sample), kPersistChunk);
-                b = __shfl_sync(0xffffffffu, b, 0);
-                if (b >= end) {
-                    exhausted = true;
-                    break;
-                }
-                cbase = b;
-                cleft = (end - b < kPersistChunk) ? (uint32_t)(end - b) : kPersistChunk;
-                // The pass of the chunk's first sample, looked up once for the warp.
-                uint32_t cj = 0;
-                if (lane == 0) cj = find_job(A.jobs, A.job_cap, job_lo, job_hi, b);
-                cjob = __shfl_sync(0xffffffffu, cj, 0);
-                const WfJob& CJ = A.jobs[cjob];
-                cjob_end = CJ.first + (uint64_t)CJ.count;
-            }
-            const uint32_t n = min((uint32_t)__popc(need), cleft);
-            const uint32_t rank = (uint32_t)__popc(need & lt);
-            const bool mine = ((need >> lane) & 1u) && rank < n;
-            if (mine) {
-                const uint64_t s = cbase + rank;
-                job = (s < cjob_end) ? cjob : find_job(A.jobs, A.job_cap, job_lo, job_hi, s);
-                const WfJob& J = A.jobs[job];
-                local = J.local_base + (uint32_t)(s - J.first);
-                const pt_push& pc = J.pc;
-                const int W = pc.resolution[0], H = pc.resolution[1];
-                const uint32_t npix = (uint32_t)W * (uint32_t)H;
-                const uint32_t k = local / npix, pix = local % npix;
-                const uint32_t xx = pix % (uint32_t)W, yy = (uint32_t)H - pix / (uint32_t)W;
-                const float uvx = (2.0f * (float)xx - (float)W) / (float)H;
-                const float uvy = (2.0f * (float)yy - (float)H) / (float)H;
-                const CamInfo cam = J.cam;
-                start_sample(ps, ONE ? *S1 : *J.scene, pc, cam, xx, yy, uvx, uvy, (int)k);
-                shadow = false;
-                sign.set = 0u;
-                active = true;
-            }
-            cbase += n;
-            cleft -= n;
-            need = __ballot_sync(0xffffffffu, !active);
-        }
-        if (exhausted && __ballot_sync(0xffffffffu, active) == 0) break;
-        bool finished = false;
-        if (active) {
-            const WfJob& J = A.jobs[job];
-            const KScene& S = ONE ? *S1 : *J.scene;
-            const int depth = J.pc.pathLength;
-            Hit h;
-            h.hitdist = PT_MAXDIST;
-            h.normal = f3(0.0f, 0.0f, 0.0f);
-            h.materialID = 0.0f;
-            h.lightID = -1.0f;
-            int objectID = -1;
-            intersect_all<FEAT>(S, ONE ? sphS : S.objects, ps.org, shadow ? ps.shDir : ps.dir, h, objectID, shadow, ps.shObj, sign);
-            if (!shadow) sign.set = 0u;  // shading moves the origin
-            const StepResult r = shadow ? shade_shadow<false>(ps, S, objectID, depth)
-                                        : shade_primary<false>(ps, S, h, objectID, depth);
-            shadow = (r == STEP_SHADOW);
-            if (r == STEP_TERMINATED) {
-                const float3 col = sample_color(ps, S, J.cie);
-                if (pt_check(A, local - J.local_base, J.count, PT_CHECK_SAMPLE))
-                    J.colors[local] = make_float4(col.x, col.y, col.z, 0.0f);
-                finished = true;
-                active = false;
-            }
-        }
-        count_finished(A.jobs, job, finished);
-    }
-}
-
-template <int FEAT>
-__global__ void __launch_bounds__(kPersistThreads) wf_persist(const __grid_constant__ WfArgs A) {
-    persist_paths<FEAT, false>(A, nullptr);
-}
-
-template <int FEAT>
-__global__ void __launch_bounds__(kPersistThreads)
-    wf_persist_one(const __grid_constant__ WfArgs A, const __grid_constant__ KScene S1) {
-    persist_paths<FEAT, true>(A, &S1);
-}
-
 __global__ void wf_book(const __grid_constant__ WfArgs A) {
     WfCounters& C = *A.counters;
     const uint32_t pool = A.pool_size;
@@ -617,7 +440,7 @@ __global__ void wf_init(WfCounters* __restrict__ Cp, uint32_t* __restrict__ q_fr
         C.iterations = 0;
         C.live = 0;
         C.job_lo = C.job_hi = 0;
-        C.pk_end = 0;
+        C.pk_begin = C.pk_end = 0;
         C.check_site = 0;
         C.check_index = 0;
     }
@@ -705,53 +528,6 @@ cudaError_t PTK_WF(ptk_wavefront_launch_iteration)(const WfArgs* a, bool trace, 
     return cudaGetLastError();
 }
 
-namespace {
-
-// Blocks of a persistent kernel that fit on one SM at once, cached.
-template <int FEAT, bool ONE>
-int persist_blocks() {
-    static int cache = 0;
-    if (cache) return cache;
-    int n = 0;
-    const void* k = ONE ? reinterpret_cast<const void*>(wf_persist_one<FEAT>)
-                        : reinterpret_cast<const void*>(wf_persist<FEAT>);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kPersistThreads, 0) != cudaSuccess || n < 1) n = 1;
-    cache = n;
-    return n;
-}
-
-template <int FEAT>
-void launch_persist(const WfArgs* a, int sms, const KScene* one_scene, cudaStream_t stream) {
-    if (one_scene) {
-        wf_persist_one<FEAT><<<sms * persist_blocks<FEAT, true>(), kPersistThreads, 0, stream>>>(*a, *one_scene);
-    } else {
-        wf_persist<FEAT><<<sms * persist_blocks<FEAT, false>(), kPersistThreads, 0, stream>>>(*a);
-    }
-}
-
-}  // namespace
-
-cudaError_t PTK_WF(ptk_persist_launch)(const WfArgs* a, int variant, int sms, uint64_t budget,
-                                       const KScene* one_scene, cudaStream_t stream) {
-    wf_persist_setup<<<1, 1, 0, stream>>>(*a, budget);
-    switch (variant) {
-        case 0: launch_persist<0>(a, sms, one_scene, stream); break;
-        case PT_FEAT_BOX: launch_persist<PT_FEAT_BOX>(a, sms, one_scene, stream); break;
-        case PT_FEAT_ANALYTIC: launch_persist<PT_FEAT_ANALYTIC>(a, sms, one_scene, stream); break;
-        default: launch_persist<PT_FEAT_ALL>(a, sms, one_scene, stream); break;
-    }
-    return cudaGetLastError();
-}
-
-int PTK_WF(ptk_persist_blocks_per_sm)(int variant) {
-    switch (variant & 15) {
-        case 0: return persist_blocks<0, false>();
-        case PT_FEAT_BOX: return persist_blocks<PT_FEAT_BOX, false>();
-        case PT_FEAT_ANALYTIC: return persist_blocks<PT_FEAT_ANALYTIC, false>();
-        default: return persist_blocks<PT_FEAT_ALL, false>();
-    }
-}
-
 cudaError_t PTK_WF(ptk_wavefront_launch_resolve)(const WfArgs* a, uint32_t job, const pt_push* pc, float4* accum,
                                          const float4* colors, cudaStream_t stream) {
     (void)a;
@@ -760,6 +536,11 @@ cudaError_t PTK_WF(ptk_wavefront_launch_resolve)(const WfArgs* a, uint32_t job, 
     wf_resolve<<<(npix + kStageThreads - 1) / kStageThreads, kStageThreads, 0, stream>>>(*pc, accum, colors);
     return cudaGetLastError();
 }
+
+// pt_persist.cu
+cudaError_t PTK_WF(ptk_persist_launch)(const WfArgs* a, int variant, int sms, uint64_t budget,
+                                       const KScene* one_scene, cudaStream_t stream);
+int PTK_WF(ptk_persist_blocks_per_sm)(int variant);
 
 extern const WfKernelSet PTK_WF(ptk_wavefront_kernel_set);
 const WfKernelSet PTK_WF(ptk_wavefront_kernel_set) = {

@@ -62,7 +62,8 @@ struct WfCounters {
     uint32_t live;         // slots holding a path (pool - n_free)
     uint32_t job_lo;       // oldest pass that may still hold unfinished samples
     uint32_t job_hi;       // passes added so far
-    uint64_t pk_end;       // persistent mode: end of the sample range of the current launch
+    uint64_t pk_begin;     // persistent mode: the sample range of the current launch
+    uint64_t pk_end;
     uint32_t n_shadow[2];  // shadow-ray results to shade (current, next)
     // Kernels built with PT_DEBUG_CHECKS: the first index check that failed
     // since the last reset (PT_CHECK_* site, 0: none) and the index it saw.
@@ -98,7 +99,7 @@ struct WfArgs {
     int refill_min;    // idle lanes a march warp gathers before it refills them at once
     int drain_lanes;   // a drained march warp with fewer rays suspends them (0: never)
     int march_inner;   // SDF evaluations per lane between a march warp's refills and queue appends
-    int persist_refill;  // idle lanes a persistent warp gathers before starting new samples together
+    int persist_refill;  // ended paths a persistent warp gathers before starting new samples together
 };
 
 // Host side (not seen by the run-time compiled program, pt_jit.cu).
