@@ -75,11 +75,73 @@ PT_DI int path_class(const KScene& S, const Hit& h, bool shadow) {
     return (xm && xm->type >= PT_BSDF_MIRROR) ? PC_SPECULAR : PC_DIFFUSE;
 }
 
+// POOL: takes queue entry e of the staged engine over into slot state q and
+// ps.  A marching ray (`march`) is intersected again from its origin, whatever
+// it had marched (the result is the same): returns PC_COUNT, with r telling
+// its kind.  A hit or a shadow result (`result`) is ready to shade: returns
+// its class.  -1: an index check failed.
+PT_DI int load_staged(const WfArgs& A, const PoolView& v, uint32_t e, bool march, bool result, PathState& ps,
+                      float4& contrib, float4* q, uint32_t& local, uint32_t& job, StepResult& r) {
+    const uint32_t slot = result ? (e & kQueueSlotMask) : e;
+    if (!pt_check(A, slot, A.pool_size, PT_CHECK_QUEUE_SLOT)) return -1;
+    const uint4 w = v.s8[slot];
+    job = word_job(w.w);
+    if (!pt_check(A, job, A.job_cap, PT_CHECK_JOB)) return -1;
+    const KScene& S = *A.jobs[job].scene;
+    const float4 a = v.s0[slot], b = v.s1[slot];
+    const bool shadow = result || (march && (w.y & kShadowFlag) != 0);
+    ps.org = f3(a.x, a.y, a.z);
+    ps.mis = a.w;
+    ps.dir = f3(b.x, b.y, b.z);
+    ps.l = v.s7[slot];
+    ps.seed = w.x;
+    ps.bounce = (int)(w.y & kBounceMask);
+    ps.medium = (int)((w.y >> kMediumShift) & 3u);
+    ps.shObj = word_shobj(w.w);
+    local = w.z;
+    if (!shadow && ps.bounce == 0) {  // not stored for a first ray (store_new_sample)
+        ps.rr = f4s(1.0f);
+        ps.radiance = f4s(0.0f);
+    } else {
+        ps.rr = v.s5[slot];
+        ps.radiance = v.s6[slot];
+    }
+    if (shadow) contrib = v.s3[slot];
+    q[2] = ps.l;
+    r = shadow ? STEP_SHADOW : STEP_CONTINUE;
+    if (march) {
+        if (shadow) {
+            const float4 d = v.s2[slot];
+            ps.shDir = f3(d.x, d.y, d.z);
+        }
+        return PC_COUNT;
+    }
+    const float4 h0 = v.h0[slot], h1 = v.h1[slot];
+    const float4 ids = result ? make_float4(__int_as_float(ps.shObj),
+                                            (e & kQueueSdfHit) ? __int_as_float(-2) : h0.w, 0.0f, 0.0f)
+                              : h0;
+    Hit h;
+    h.hitdist = h0.x;
+    h.normal = f3(h1.x, h1.y, h1.z);
+    h.materialID = h0.y;
+    h.lightID = h0.z;
+    q[0] = a;
+    q[1] = make_float4(b.x, b.y, b.z, __uint_as_float(w.x));
+    q[3] = ps.radiance;
+    q[4] = ps.rr;
+    q[5] = result ? contrib : make_float4(h0.x, h1.x, h1.y, h1.z);
+    q[6] = make_float4(result ? ids.x : h0.y, result ? ids.y : h0.z, __uint_as_float(local),
+                       __uint_as_float(bounce_word(ps)));
+    return path_class(S, h, result);
+}
+
 // The persistent path loop.  ONE: every sample of the launch belongs to one
 // pass, whose scene S1 is the launch's parameter (the constant bank, as
 // for the megakernel); otherwise each lane reads its pass's scene through
 // the pass's pointer.
-template <int FEAT, bool ONE>
+// POOL: the paths are those a staged engine has in flight (its queues of the
+// coming iteration) instead of new samples; see wf_finish.
+template <int FEAT, bool ONE, bool POOL>
 PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
     extern __shared__ __align__(16) unsigned char persist_smem[];
     PersistShared& sh = *reinterpret_cast<PersistShared*>(persist_smem);
@@ -93,13 +155,17 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
     }
     float4* const st = sh.state[warp];
     uint32_t* const jobs = sh.job[warp];
-    const uint64_t end = C.pk_end;
+    const uint32_t cur = C.cur, nm = C.n_march[cur], np = C.n_shade[cur], ns = C.n_shadow[cur];  // POOL
+    const PoolView pool = view(A);
+    const uint64_t end = POOL ? (uint64_t)nm + np + ns : C.pk_end;
     const uint32_t job_lo = C.job_lo, job_hi = C.job_hi;
     // A small launch gives every warp its share at once: no more slots than
     // that, and chunks that leave something for the others.
-    const uint64_t share = (end - C.pk_begin) / ((uint64_t)gridDim.x * kPersistWarps);
-    const int slots = share >= (uint64_t)kPersistSlots ? kPersistSlots : (share < 32 ? 32 : (int)((share + 31) / 32 * 32));
-    const uint32_t chunk = share >= 8 * kPersistChunk ? kPersistChunk : (share < 128 ? 32u : (uint32_t)(share / 128 * 32));
+    const uint64_t share = (end - (POOL ? 0 : C.pk_begin)) / ((uint64_t)gridDim.x * kPersistWarps);
+    // A staged engine's last paths are spread over every warp: their time is
+    // the longest path's, and a warp steps as long as its longest march.
+    const int slots = POOL ? min(kPersistSlots, (int)share + 1) : share >= (uint64_t)kPersistSlots ? kPersistSlots : (share < 32 ? 32 : (int)((share + 31) / 32 * 32));
+    const uint32_t chunk = POOL ? min(32u, (uint32_t)share + 1) : share >= 8 * kPersistChunk ? kPersistChunk : (share < 128 ? 32u : (uint32_t)(share / 128 * 32));
     int count[PC_COUNT] = {0, 0, 0, 0};  // warp-uniform: the lists' lengths
     for (int i = lane; i < slots; i += 32) sh.list[warp][PC_END][i] = (uint16_t)(i | (PE_START << 8));
     count[PC_END] = slots;
@@ -143,6 +209,9 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
         PathState ps;
         StepResult r = STEP_TERMINATED;
         bool coloured = false;
+        float4 contrib = f4s(0.0f);
+        int next = -1, next_end = PE_HIT;
+        bool restored = false;  // POOL: taken over from the staged engine this trip
         if (live && ends != PE_START) {
             const float4 q0 = q[0], q1 = q[1], q5 = q[5], q6 = q[6];
             job = jobs[slot];
@@ -192,7 +261,9 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
             while (need && !exhausted) {
                 if (cleft == 0) {
                     unsigned long long b = 0;
-                    if (lane == 0) b = atomicAdd(reinterpret_cast<unsigned long long*>(&C.next_sample), chunk);
+                    if (lane == 0)
+                        b = POOL ? (unsigned long long)atomicAdd(&C.march_cursor, chunk)
+                                 : atomicAdd(reinterpret_cast<unsigned long long*>(&C.next_sample), chunk);
                     b = __shfl_sync(0xffffffffu, b, 0);
                     if (b >= end) {
                         exhausted = true;
@@ -200,6 +271,7 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
                     }
                     cbase = b;
                     cleft = (end - b < chunk) ? (uint32_t)(end - b) : chunk;
+                    if constexpr (POOL) continue;
                     // The pass of the chunk's first sample, looked up once for the warp.
                     uint32_t cj = 0;
                     if (lane == 0) cj = find_job(A.jobs, A.job_cap, job_lo, job_hi, b);
@@ -211,16 +283,28 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
                 const uint32_t rank = (uint32_t)__popc(need & lt);
                 if (((need >> lane) & 1u) && rank < take) {
                     const uint64_t s = cbase + rank;
+                    started = true;
+                    if constexpr (POOL) {
+                        const uint32_t i = (uint32_t)s;
+                        const uint32_t e = i < nm        ? A.q_march[cur][i]
+                                           : i < nm + np ? A.q_shade[cur][i - nm]
+                                                         : A.q_shadow[cur][i - nm - np];
+                        next = load_staged(A, pool, e, i < nm, i >= nm + np, ps, contrib, q, local, job, r);
+                        restored = next >= 0;
+                    } else {
                     job = (s < cjob_end) ? cjob : find_job(A.jobs, A.job_cap, job_lo, job_hi, s);
                     local = A.jobs[job].local_base + (uint32_t)(s - A.jobs[job].first);
-                    started = true;
+                    }
                 }
                 cbase += take;
                 cleft -= take;
                 need = __ballot_sync(0xffffffffu, live && !started);
             }
             live = started;
-            if (live) {
+            if constexpr (POOL) {
+                live = restored;
+                if (live) jobs[slot] = job;
+            } else if (live) {
                 const WfJob& J = A.jobs[job];
                 const pt_push& pc = J.pc;
                 const int W = pc.resolution[0], H = pc.resolution[1];
@@ -237,8 +321,9 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
             }
         }
         // The ray each path goes on with, and the class of its next step.
-        int next = -1, next_end = PE_HIT;
-        if (live) {
+        if (POOL && live && restored && next < PC_COUNT) {
+            // a staged hit or shadow result: its state is in place
+        } else if (live) {
             q[3] = ps.radiance;
             const uint32_t flags = bounce_word(ps);
             if (r == STEP_TERMINATED) {
@@ -251,8 +336,8 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
                 q[0] = make_float4(ps.org.x, ps.org.y, ps.org.z, ps.mis);
                 q[1] = make_float4(ps.dir.x, ps.dir.y, ps.dir.z, __uint_as_float(ps.seed));
                 // a shadow ray's NEE term and the next throughput, made now (shade_shadow_made)
-                q[4] = shadow ? bounce_throughput(ps) : ps.rr;
-                if (shadow) q[5] = shadow_contribution(ps, S);
+                q[4] = (shadow && !(POOL && restored)) ? bounce_throughput(ps) : ps.rr;
+                if (shadow) q[5] = (POOL && restored) ? contrib : shadow_contribution(ps, S);
                 Hit h;
                 h.hitdist = PT_MAXDIST;
                 h.normal = f3(0.0f, 0.0f, 0.0f);
@@ -281,18 +366,41 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
 
 template <int FEAT>
 __global__ void __launch_bounds__(kPersistThreads, FEAT == PT_FEAT_ALL ? 4 : 5) wf_persist(const __grid_constant__ WfArgs A) {
-    persist_paths<FEAT, false>(A, nullptr);
+    persist_paths<FEAT, false, false>(A, nullptr);
 }
 
 template <int FEAT>
 __global__ void __launch_bounds__(kPersistThreads, FEAT == PT_FEAT_ALL ? 4 : 5)
     wf_persist_one(const __grid_constant__ WfArgs A, const __grid_constant__ KScene S1) {
-    persist_paths<FEAT, true>(A, &S1);
+    persist_paths<FEAT, true, false>(A, &S1);
 }
 
 }  // namespace
 
 namespace {
+
+// The last paths of a staged engine, run to their ends here.  Staged, every
+// ray of a path waits for the slowest march of each iteration (64 steps, 25 us
+// of launches): with few paths left an iteration costs the same 60 to 100 us
+// however few, about 5 ms from the last new sample to the last colour on the
+// shipped scenes.  Here a path's steps follow one another.
+__global__ void __launch_bounds__(kPersistThreads, 4) wf_finish(const __grid_constant__ WfArgs A) {
+    persist_paths<PT_FEAT_ALL, false, true>(A, nullptr);
+}
+
+// The pool is empty again: no queue holds a slot, the free list holds all.
+__global__ void wf_finish_done(const __grid_constant__ WfArgs A) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < A.pool_size) A.q_free[i] = i;
+    if (i == 0) {
+        WfCounters& C = *A.counters;
+        C.n_march[C.cur] = C.n_shade[C.cur] = C.n_shadow[C.cur] = 0;
+        C.n_free = A.pool_size;
+        C.live = 0;
+        C.march_cursor = 0;
+        C.iterations += 1;
+    }
+}
 
 // Blocks of a persistent kernel that fit on one SM at once, cached.
 template <int FEAT, bool ONE>
@@ -343,4 +451,22 @@ int PTK_WF(ptk_persist_blocks_per_sm)(int variant) {
         case PT_FEAT_ANALYTIC: return persist_blocks<PT_FEAT_ANALYTIC, false>();
         default: return persist_blocks<PT_FEAT_ALL, false>();
     }
+}
+
+cudaError_t PTK_WF(ptk_wavefront_finish)(const WfArgs* a, int sms, cudaStream_t stream) {
+    static int blocks = 0;
+    if (!blocks) {
+        const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(wf_finish),
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PersistShared));
+        if (e != cudaSuccess) return e;
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_finish, kPersistThreads, sizeof(PersistShared)) !=
+                cudaSuccess ||
+            n < 1)
+            n = 1;
+        blocks = n;
+    }
+    wf_finish<<<sms * blocks, kPersistThreads, sizeof(PersistShared), stream>>>(*a);
+    wf_finish_done<<<(a->pool_size + 255) / 256, 256, 0, stream>>>(*a);
+    return cudaGetLastError();
 }

@@ -142,6 +142,11 @@ constexpr int kPersistThreads = 128;
 cudaError_t ptk_wavefront_launch_resolve(const WfArgs* a, uint32_t job, const pt_push* pc, float4* accum,
                                          const float4* colors, cudaStream_t stream);
 
+// Between iterations of a staged engine with no sample left to start: runs
+// every path in flight to its end in one launch and empties the pool.  For
+// scenes of built-in SDF plug-ins.
+cudaError_t ptk_wavefront_finish(const WfArgs* a, int sms, cudaStream_t stream);
+
 // The launch functions above as a set, for the engine to switch between the
 // default build of the wavefront kernels and the checked one.
 struct WfKernelSet {
@@ -152,6 +157,7 @@ struct WfKernelSet {
     cudaError_t (*persist)(const WfArgs*, int, int, uint64_t, const KScene*, cudaStream_t);
     int (*persist_blocks_per_sm)(int);
     cudaError_t (*resolve)(const WfArgs*, uint32_t, const pt_push*, float4*, const float4*, cudaStream_t);
+    cudaError_t (*finish)(const WfArgs*, int, cudaStream_t);
 };
 // checked = false: the kernels above; true: the same kernels built with
 // PT_DEBUG_CHECKS (pt_wavefront_checked.cu): every queue, pool-slot, ring and

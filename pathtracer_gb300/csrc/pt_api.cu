@@ -49,7 +49,6 @@ struct pt_ctx {
     WfEngine* wf = nullptr;        // wavefront driver (created on first use, grows with the dispatch)
     WfEngine* persist = nullptr;   // the persistent kernel's, for scenes without SDFs (created on first use)
     bool staged_knobs = false;     // the caller set a knob of the staged engine: dispatches keep to it
-    cudaStream_t last_stream = nullptr;  // stream of the last persistent dispatch
     // More engines, on streams of their own, take equal shares of a large
     // dispatch's samples (pt_set_wavefront_engines); `fork` orders them after
     // the context's stream, `join` the resolve after them.
@@ -117,6 +116,12 @@ cudaError_t sync_device_scene(pt_ctx* ctx) {
 }
 
 }  // namespace
+
+// Samples up to which a dispatch of built-in SDFs takes the persistent kernel.
+// Measured on GB300, persistent and staged, ms: shipped mandelbulb 64x64x1
+// 1.55 and 2.19, 320x180x1 2.28 and 3.66, 320x180x4 2.61 and 4.54, 512x512x4
+// 8.2 and 6.8; menger + terrain 160x90x1 1.61 and 3.27, 320x180x2 2.91 and 3.87.
+constexpr uint64_t kSmallDispatch = 1ull << 18;
 
 static int dispatch_wavefront(pt_ctx* ctx, const pt_push* push);
 static int dispatch_persistent(pt_ctx* ctx, const pt_push* push);
@@ -373,12 +378,17 @@ int pt_dispatch(pt_ctx* ctx, const pt_push* push) {
     }
     if (ctx->engine == PT_ENGINE_WAVEFRONT && push->pathLength > 0) {
         // A scene without SDFs has nothing for the staged kernels to sort:
-        // its paths stay on chip in the persistent kernel (1024x1024x16
-        // sphere scene, 256x256x16 Cornell box: see dispatch_persistent).
+        // its paths stay on chip in the persistent kernel (dispatch_persistent).
         // Whatever asks for the staged kernels themselves gets them: traces,
         // stage times, index checks, a drain limit or a staged knob.
         const bool plain_call = !trace && !ctx->stage_timing && !ctx->device_checks && ctx->drain_limit == 0;
-        if (P.s.meta.n[5] == 0 && plain_call && !ctx->staged_knobs) return dispatch_persistent(ctx, push);
+        // So does a dispatch of few samples of built-in SDFs, whose time is the
+        // longest path's: the staged engine makes every path wait for the
+        // slowest march of each step (measured: kSmallDispatch).
+        const uint64_t total = (uint64_t)push->resolution[0] * (uint64_t)push->resolution[1] *
+                               (uint64_t)push->samplesPerFrame;
+        const bool on_chip = P.s.meta.n[5] == 0 || (ctx->custom.empty() && total <= kSmallDispatch);
+        if (on_chip && plain_call && !ctx->staged_knobs) return dispatch_persistent(ctx, push);
         return dispatch_wavefront(ctx, push);
     }
     ctx->last_launches = 1;
@@ -660,7 +670,14 @@ void* pt_stream(pt_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
 
 int pt_set_stream(pt_ctx* ctx, void* stream) {
     if (!ctx) return PT_ERR_INVALID;
-    ctx->stream = stream ? (cudaStream_t)stream : ctx->own_stream;
+    const cudaStream_t s = stream ? (cudaStream_t)stream : ctx->own_stream;
+    if (s != ctx->stream) {
+        // The scene's device copy, the colour buffer and the engines belong to
+        // the last dispatch until it is done.
+        PT_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
+        PT_CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->done, 0));
+    }
+    ctx->stream = s;
     return PT_OK;
 }
 
@@ -691,19 +708,14 @@ const char* pt_last_error(pt_ctx* ctx) {
 
 }  // extern "C"
 
-// A dispatch of a scene without SDFs: one pass on the persistent kernel, in
-// one launch, then the resolve.  Nothing is read back, so the call returns
+// A dispatch of a scene without SDFs, or of few samples: one pass on the
+// persistent kernel, in one launch, then the resolve.  Nothing is read back, so the call returns
 // with the work queued, like the megakernel's; measured on GB300 against the
-// staged engine: Cornell box 256x256 1.61 -> 0.45 ms at 16 spp, 0.61 -> 0.09
-// ms at 1.
+// staged engine: Cornell box 256x256 at 1 spp 640 -> 112 us a frame.
 static int dispatch_persistent(pt_ctx* ctx, const pt_push* push) {
     const uint64_t total = (uint64_t)push->resolution[0] * (uint64_t)push->resolution[1] *
                            (uint64_t)push->samplesPerFrame;
     if (total >= (1ull << 32)) return fail(ctx, PT_ERR_INVALID, "pt_dispatch: more than 2^32 samples in one dispatch");
-    // The pass's colours, counters and job entry belong to the dispatch before
-    // until it is done: on another stream, wait for it.
-    if (ctx->last_stream && ctx->last_stream != ctx->stream)
-        PT_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream, ctx->done, 0));
     if (!ctx->persist) {
         WfEngine* E = new (std::nothrow) WfEngine();
         if (!E) return fail(ctx, PT_ERR_OOM, "pt_dispatch: out of host memory");
@@ -746,7 +758,6 @@ static int dispatch_persistent(pt_ctx* ctx, const pt_push* push) {
     ctx->last_iterations = 1;
     ctx->last_launches = E.kernel_launches - launches0;
     PT_CUDA_TRY(ctx, cudaEventRecord(ctx->done, ctx->stream));
-    ctx->last_stream = ctx->stream;
     return PT_OK;
 }
 
@@ -760,6 +771,8 @@ static int dispatch_wavefront(pt_ctx* ctx, const pt_push* push) {
     if (total64 >= (1ull << 32)) return fail(ctx, PT_ERR_INVALID, "pt_dispatch: more than 2^32 samples in one dispatch");
     const uint32_t total = (uint32_t)total64;
     const bool trace = ctx->trace.events || ctx->trace.nevents || ctx->trace.colors;
+    const bool finish = !trace && !ctx->stage_timing && !ctx->device_checks && ctx->drain_limit == 0 &&
+                        !ctx->staged_knobs && ctx->custom.empty();
     int n = 1;
     if (!trace && !ctx->stage_timing) {
         const uint64_t fit = total64 / (2ull * ctx->pool_cap);
@@ -832,6 +845,7 @@ static int dispatch_wavefront(pt_ctx* ctx, const pt_push* push) {
         E.set_march_budget(ctx->march_budget);
         E.set_tuning(ctx->refill_min, ctx->drain_lanes, ctx->blocks_per_sm, ctx->march_inner);
         if (e == 0 && E.stage_timing != ctx->stage_timing) PT_CUDA_TRY(ctx, E.set_stage_timing(ctx->stage_timing));
+        E.finish_at = finish ? finish_threshold(total64) : 0u;
         E.args.trace = e == 0 ? ctx->trace : KTrace{nullptr, nullptr, nullptr, 0};
         PT_CUDA_TRY(ctx, E.reset());
         uint32_t idx = 0;

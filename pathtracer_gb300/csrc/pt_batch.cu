@@ -191,6 +191,7 @@ cudaError_t ensure_engine(pt_batch* b, int e) {
     b->engine[e].set_persistent(e == kPersistent);
     b->engine[e].args.persist_refill = b->persist_refill;
     b->engine[e].set_checks(b->device_checks);
+    b->engine[e].finish_at = e == kPersistent ? 0u : kFinishAt;  // pt_batch_run
     if (e != kPersistent) b->engine[e].set_march_kernel(staged_march_kernel(b));
     b->engine_live[e] = true;
     return cudaSuccess;
@@ -916,13 +917,31 @@ int pt_batch_run(pt_batch* b, uint64_t max_iterations) {
     uint64_t iters = 0;
     int chunk = 8;
     int ids[256];
+    uint64_t began[kEngines] = {0, 0, 0};  // samples started when a staged engine's counters were last read
     while (pt_batch_pending(b) > 0) {
         if (iters >= max_iterations) return bfail(b, PT_ERR_KERNEL, "pt_batch_run: passes did not finish");
         int nc = 0;
         const int rc = pt_batch_step(b, chunk, ids, 256, &nc);
         if (rc != PT_OK) return rc;
         iters += (uint64_t)chunk;
-        if (chunk < 64) chunk *= 2;
+        // A staged engine whose last samples are under way finishes them in one
+        // launch (built-in SDFs); the next step reports them.
+        int next = 0;
+        for (int e : {kStaged, kStaged2}) {
+            WfEngine& E = b->engine[e];
+            if (!b->engine_live[e] || E.njobs <= E.lo || !b->custom.empty() || b->device_checks) continue;
+            WfCounters c;
+            PT_B_TRY(b, E.read_counters(&c));
+            if (E.can_finish(c)) PT_B_TRY(b, E.finish());
+            const int n = E.next_chunk(c, c.next_sample - began[e], chunk);
+            next = next == 0 || n < next ? n : next;
+            began[e] = c.next_sample;
+        }
+        if (next > 0) {
+            chunk = next;
+        } else if (chunk < 64) {
+            chunk *= 2;
+        }
     }
     PT_B_TRY(b, cudaStreamSynchronize(b->stream));
     return PT_OK;

@@ -353,6 +353,21 @@ cudaError_t WfEngine::resolve(uint32_t j, cudaStream_t on) {
     return kernels->resolve(&args, j % max_jobs, &J.pc, J.accum, J.colors, on ? on : stream);
 }
 
+cudaError_t WfEngine::finish() {
+    kernel_launches += 2;
+    return kernels->finish(&args, sms, stream);
+}
+
+int WfEngine::next_chunk(const WfCounters& c, uint64_t started, int ran) const {
+    if (finish_at == 0) return ran < 64 ? 2 * ran : 64;  // (doubling from the caller's first chunk)
+    // Read again about when the last sample starts, then every four
+    // iterations: the sooner the few last paths are finished together.
+    const uint64_t left = c.total - c.next_sample;
+    if (left == 0 || started == 0) return 4;
+    const uint64_t n = left * (uint64_t)ran / started + 1;
+    return n >= 64 ? 64 : n <= 4 ? 4 : (int)((n + 3) / 4 * 4);
+}
+
 cudaError_t wf_drain_many(WfEngine* const* e, int n, uint64_t max_iterations) {
     constexpr int kMax = 8;
     if (n < 1 || n > kMax) return cudaErrorInvalidValue;
@@ -364,9 +379,11 @@ cudaError_t wf_drain_many(WfEngine* const* e, int n, uint64_t max_iterations) {
     int chunk[kMax];
     uint64_t iter[kMax];
     bool done[kMax];
+    uint64_t began[kMax];  // samples started when the counters were last read
     for (int i = 0; i < n; i++) {
         chunk[i] = 8;
         iter[i] = 8;
+        began[i] = 0;
         done[i] = false;
         EN_TRY(e[i]->run(chunk[i], false));
     }
@@ -382,7 +399,14 @@ cudaError_t wf_drain_many(WfEngine* const* e, int n, uint64_t max_iterations) {
                 continue;
             }
             if (iter[i] > max_iterations) return cudaErrorTimeout;
-            if (chunk[i] < 64) chunk[i] *= 2;
+            if (e[i]->can_finish(c)) {
+                EN_TRY(e[i]->finish());
+                done[i] = true;
+                left--;
+                continue;
+            }
+            chunk[i] = e[i]->next_chunk(c, c.next_sample - began[i], chunk[i]);
+            began[i] = c.next_sample;
             EN_TRY(e[i]->run(chunk[i], false));
             iter[i] += (uint64_t)chunk[i];
         }
@@ -399,8 +423,9 @@ cudaError_t WfEngine::drain(bool trace, uint64_t max_iterations) {
         }
         return read_counters(host_counters);
     }
-    uint64_t iter = 0;
-    int chunk = 8;
+    uint64_t iter = 0, began = 0;
+    // a dispatch that starts every sample at once is read back sooner
+    int chunk = finish_at > 0 && total <= (uint64_t)pool ? 4 : 8;
     WfCounters c;
     for (;;) {
         EN_TRY(run(chunk, trace));
@@ -411,6 +436,8 @@ cudaError_t WfEngine::drain(bool trace, uint64_t max_iterations) {
         // stop here; the caller reports it (check_failed).
         if (c.check_site != PT_CHECK_NONE) return cudaSuccess;
         if (iter > max_iterations) return cudaErrorTimeout;
-        if (chunk < 64) chunk *= 2;
+        if (!trace && can_finish(c)) return finish();
+        chunk = next_chunk(c, c.next_sample - began, chunk);
+        began = c.next_sample;
     }
 }

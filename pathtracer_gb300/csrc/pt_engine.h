@@ -69,6 +69,18 @@ inline const char* pt_check_site_name(uint32_t site) {
     }
 }
 
+// Paths in flight at which a staged engine's drain hands the rest to one
+// launch (WfEngine::finish_at).  Measured on GB300, ms with 2^14, 2^16 and no
+// such launch: shipped mandelbulb 777x431x16 9.9, 10.3, 11.2; menger + terrain
+// 640x360x4 9.2, 10.0, 11.9; feature mix 641x359x2 (460 K samples) 2.95, 2.65,
+// 3.5: a dispatch of few samples is all tail, and hands over sooner.
+constexpr uint32_t kFinishAt = 1u << 14;
+constexpr uint32_t kFinishAtSmall = 1u << 16;
+constexpr uint64_t kFinishSmallTotal = 1ull << 19;
+inline uint32_t finish_threshold(uint64_t samples) {
+    return samples <= kFinishSmallTotal ? kFinishAtSmall : kFinishAt;
+}
+
 struct WfEngine;
 // Drains n (1..8) staged engines on different streams, each relaunched as
 // soon as its last chunk of iterations has been read back, so that one
@@ -98,7 +110,7 @@ struct WfEngine {
     bool owns_host_counters = false;
     // Graph replay of `graph_chunk` iterations (engines that allocate only).
     bool use_graph = false;
-    int graph_chunk = 8;
+    int graph_chunk = 4;
     cudaGraphExec_t graph = nullptr;
     // Persistent mode: each iteration is one launch of the persistent path
     // kernel over the next `persist_budget` samples instead of one pass of
@@ -110,6 +122,10 @@ struct WfEngine {
     // its scene in the constant bank) instead of sharing one with the next.
     static constexpr uint64_t kPersistOnePassMin = 1ull << 20;
     uint64_t persist_issued = 0;  // samples covered by launches so far
+    // Staged: once no sample is left to start and at most this many paths are
+    // in flight, drain() runs them to their ends in one launch (finish);
+    // 0: never (scenes with run-time compiled SDFs, traces).
+    uint32_t finish_at = 0;
     // Stage timing (off by default): every iteration is launched without the
     // graph, bracketed by events; stage_ms accumulates device milliseconds.
     bool stage_timing = false;
@@ -171,6 +187,17 @@ struct WfEngine {
     void retire(uint32_t new_lo);
     // Launches `n` iterations.
     cudaError_t run(int n, bool trace);
+    // Staged: runs every path in flight to its end in one launch.  Valid when
+    // no sample is left to start and every SDF is a built-in plug-in.
+    cudaError_t finish();
+    // Whether drain() may end with finish() now, given the counters.
+    bool can_finish(const WfCounters& c) const {
+        return finish_at > 0 && c.next_sample == c.total && c.live > 0 && c.live <= finish_at &&
+               c.check_site == PT_CHECK_NONE;
+    }
+    // Iterations to run before the counters are read again, given what the
+    // last `ran` of them started.
+    int next_chunk(const WfCounters& c, uint64_t started, int ran) const;
     // Stage timing on or off (clears the totals).
     cudaError_t set_stage_timing(bool on);
     // Reads the counters (synchronises the stream).
