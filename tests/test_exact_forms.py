@@ -205,3 +205,83 @@ def test_culled_spheres_are_never_hit(tmp_path, scale, kind):
     assert not (out == 3).any()
     if kind == "any" and scale <= 300.0:
         assert (out == 2).mean() > 0.5  # the pass does leave spheres out
+
+
+BYTE_C = r"""
+#include <fenv.h>
+#include <math.h>
+#include <stdint.h>
+#include <string.h>
+static float fb(uint32_t u) { float f; memcpy(&f, &u, 4); return f; }
+static uint32_t bits(float f) { uint32_t u; memcpy(&u, &f, 4); return u; }
+/* x * 255 + 2^23 rounded down against the truncated double product, at every step-th float of [0, 1] and at the 64
+   floats on either side of each k / 255 */
+long bytes_differ(uint32_t step) {
+    long bad = 0;
+    uint32_t u;
+    int k, i;
+    const uint32_t one = bits(1.0f);
+    fesetround(FE_DOWNWARD);
+    for (u = 0; u <= one; u += step) {
+        volatile float x = fb(u), y = fmaf(x, 255.0f, 8388608.0f);
+        bad += (uint8_t)bits(y) != (uint8_t)(int)((double)x * 255.0);
+    }
+    for (k = 0; k <= 255; k++) {
+        const uint32_t c = bits((float)(k / 255.0));
+        for (i = -64; i <= 64; i++) {
+            if ((int64_t)c + i < 0 || c + i > one) continue;
+            volatile float x = fb(c + i), y = fmaf(x, 255.0f, 8388608.0f);
+            bad += (uint8_t)bits(y) != (uint8_t)(int)((double)x * 255.0);
+        }
+    }
+    fesetround(FE_TONEAREST);
+    return bad;
+}
+"""
+
+
+def test_export_byte_is_the_truncated_product(tmp_path):
+    import ctypes
+
+    src, lib = tmp_path / "b.c", tmp_path / "b.so"
+    src.write_text(BYTE_C)
+    subprocess.run([os.environ.get("CC", "gcc"), "-O1", "-std=c11", "-ffp-contract=off", "-frounding-math", "-fPIC",
+                    "-shared", "-o", str(lib), str(src), "-lm"], check=True)
+    fn = ctypes.CDLL(str(lib)).bytes_differ
+    fn.restype, fn.argtypes = ctypes.c_long, [ctypes.c_uint32]
+    assert fn(257) == 0
+
+
+EXPORT_CPP = r"""
+#include "pt_export.cuh"
+static float srgb(float x) {
+    x = (x < 0.0f) ? 0.0f : ((1.0f < x) ? 1.0f : x);
+    if (x <= 0.0031308f) return 12.92f * x;
+    return 1.055f * ptm_powf(x, 1.0f / 2.4f) - 0.055f;
+}
+/* companded values (all floats) and tonemap 3's bytes (floats not below zero, as the chain's max leaves them) */
+extern "C" long export_differs(uint32_t first, uint32_t step) {
+    long bad = 0;
+    for (uint64_t u = first; u < (1ull << 32); u += step) {
+        const float x = ptm_from_bits((uint32_t)u), a = srgb(x), b = ptx_srgb(x);
+        bad += ptm_bits(a) != ptm_bits(b) && !(a != a && b != b);
+        if (!(x < 0.0f)) bad += ptx_byte(srgb(ptm_expf(-0.25f / x))) != ptx_byte(ptx_srgb(ptx_tonemap(x, 3)));
+    }
+    return bad;
+}
+"""
+
+
+@pytest.mark.parametrize("first,step", [(0, 4099), (0x80000000, 0x7fffffff), (0x3b4d2e00, 1 << 30)])
+def test_export_forms_are_the_plain_chain(tmp_path, first, step):
+    """ptx_srgb and the exponential tonemap without their range checks: strided
+    over all floats, -0 and the companding border among them."""
+    import ctypes
+
+    src, lib = tmp_path / "e.cpp", tmp_path / "e.so"
+    src.write_text(EXPORT_CPP)
+    subprocess.run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-ffp-contract=off", "-fPIC", "-shared",
+                    "-I" + os.path.join(ROOT, "pathtracer_gb300", "csrc"), "-o", str(lib), str(src)], check=True)
+    fn = ctypes.CDLL(str(lib)).export_differs
+    fn.restype, fn.argtypes = ctypes.c_long, [ctypes.c_uint32, ctypes.c_uint32]
+    assert fn(first, step) == 0

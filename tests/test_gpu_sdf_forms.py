@@ -46,3 +46,27 @@ def test_terrain_far_out_matches_oracle(rt, x, z, engine):
         acc_g, tr_g = compare.run_gpu(ctx, push, trace_depth=depth)
     rep = compare.compare(acc_o, tr_o, acc_g, tr_g, spf)
     assert compare.passes(rep) and rep["path_match"] == 1.0, rep
+
+
+def test_device_export_bytes_match_host(rt):
+    """A large image with values on both sides of every byte's border, zeros,
+    negatives, infinities and NaN, through every tonemap."""
+    import numpy as np
+    import torch
+
+    from pathtracer_gb300 import export_rgb8, native
+
+    rng = np.random.default_rng(5)
+    W, H = 1031, 517
+    acc = np.ones((H, W, 4), np.float32)
+    acc[..., :3] = np.exp(rng.uniform(-9.0, 3.0, (H, W, 1))) * rng.uniform(0.5, 1.5, (H, W, 3))
+    acc.reshape(-1, 4)[::11, :3] *= -1.0
+    acc.reshape(-1, 4)[5::997, 0] = np.nan
+    acc.reshape(-1, 4)[6::997, 1] = np.inf
+    acc.reshape(-1, 4)[7::997, :3] = 0.0
+    d_acc, d_rgb = torch.from_numpy(acc).cuda(), torch.zeros(H * W * 3, dtype=torch.uint8, device="cuda")
+    for tm in range(4):
+        assert native.cuda().pt_export_rgb8_device(d_acc.data_ptr(), W, H, tm, d_rgb.data_ptr(), None) == native.PT_OK
+        torch.cuda.synchronize()
+        with np.errstate(all="ignore"):
+            assert np.array_equal(d_rgb.cpu().numpy().reshape(H, W, 3), export_rgb8(acc, tm)), tm
