@@ -108,6 +108,9 @@ struct PoolView {
 // writes nothing else: bit 31 an SDF hit, bits 29-30 the SDF's sign at the
 // ray's origin + 2 (0: not marched).
 constexpr uint32_t kQueueSlotMask = (1u << 28) - 1u;
+// An entry of the MARCH queues: the slot and, above it, the ray's march group.
+PT_DI uint32_t march_entry(uint32_t slot, uint32_t group) { return slot | (group << 28); }
+static_assert(kMarchGroups <= 16, "march groups must fit the four bits above a slot");
 constexpr uint32_t kQueueSdfHit = 1u << 31;
 PT_DI uint32_t shadow_entry(uint32_t slot, bool hit, float k) {
     return slot | (hit ? kQueueSdfHit : 0u) | ((k > 0.0f ? 3u : (k < 0.0f ? 1u : 2u)) << 29);
@@ -279,7 +282,7 @@ PT_DI void march_rays(const WfArgs& A) {
     WfCounters& C = *A.counters;
     const uint32_t cur = C.cur;
     const uint32_t n = C.n_march[cur];
-    const uint32_t* __restrict__ qin = A.q_march[cur];
+    const uint32_t* __restrict__ qin = A.groups > 1 ? A.q_sorted : A.q_march[cur];
     const PoolView v = view(A);
     const PoolView& M = v;
     const int lane = threadIdx.x & 31;
@@ -301,7 +304,7 @@ PT_DI void march_rays(const WfArgs& A) {
     int nnormals = 0;  // warp-uniform: records in the warp's normal stage
     const int wib = (int)(threadIdx.x >> 5);
 
-    uint32_t slot = 0;
+    uint32_t entry = 0;  // the ray's queue entry: slot and group
     const KScene* Sp = nullptr;
     int phase = MP_EMPTY;
     bool exhausted = false;
@@ -342,9 +345,10 @@ PT_DI void march_rays(const WfArgs& A) {
             if (need) {
                 const uint32_t rank = (uint32_t)__popc(mneed & ((1u << lane) - 1u));
                 const uint32_t idx = (rank < from_old) ? old_base + rank : nb + (rank - from_old);
-                if (idx < n && pt_check(A, qin[idx], A.pool_size, PT_CHECK_QUEUE_SLOT) &&
-                    pt_check(A, slot_job(v, qin[idx]), A.job_cap, PT_CHECK_JOB)) {
-                    slot = qin[idx];
+                const uint32_t e = idx < n ? qin[idx] : 0u, slot = e & kQueueSlotMask;
+                if (idx < n && pt_check(A, slot, A.pool_size, PT_CHECK_QUEUE_SLOT) &&
+                    pt_check(A, slot_job(v, slot), A.job_cap, PT_CHECK_JOB)) {
+                    entry = e;
                     const uint4 w8 = v.s8[slot];
                     Sp = A.jobs[word_job(w8.w)].scene;
                     const float4 o = v.s0[slot];
@@ -465,6 +469,7 @@ PT_DI void march_rays(const WfArgs& A) {
                     }
                 } else if (!finished && (++steps >= budget || (drain && steps >= kDrainMinSteps))) {
                     // out of budget for this launch: save the state, continue next iteration
+                    const uint32_t slot = entry & kQueueSlotMask;
                     M.m0[slot] = make_float4(t, insT, omega, prevR);
                     M.m1[slot] = make_float4(tmm.x, tmm.y, __uint_as_float(march_word(k, points, iter)),
                                              __uint_as_float(set1));
@@ -498,7 +503,7 @@ PT_DI void march_rays(const WfArgs& A) {
                     const int at = nnormals + __popc(conv & ((1u << lane) - 1u));
                     const uint64_t sp = reinterpret_cast<uint64_t>(Sp);
                     ns.at[at] = make_float4(p.x, p.y, p.z, t);
-                    ns.of[at] = make_uint4(set1, slot, (uint32_t)sp, (uint32_t)(sp >> 32));
+                    ns.of[at] = make_uint4(set1, entry & kQueueSlotMask, (uint32_t)sp, (uint32_t)(sp >> 32));
                     ns.sel[at] = hit_sel;
                     phase = MP_EMPTY;
                 }
@@ -511,16 +516,18 @@ PT_DI void march_rays(const WfArgs& A) {
                 }
             }
         } else if (finished && hit && !shadow_ray) {
+            const uint32_t slot = entry & kQueueSlotMask;
             const float3 nrm = normalize3(nv);
             const float mat = scene_sdf_material_hit(*Sp, p, set1, hit_sel);
             v.h0[slot] = make_float4(t - 1e-3f, mat, -1.0f, __int_as_float(-2));
             v.h1[slot] = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
         }
-        stage_push(A, staged[wib][0], nstaged[0], finished && !shadow_ray, slot, A.q_shade[cur], &C.n_shade[cur],
+        stage_push(A, staged[wib][0], nstaged[0], finished && !shadow_ray, entry & kQueueSlotMask,
+                   A.q_shade[cur], &C.n_shade[cur],
                    lane);
-        stage_push(A, staged[wib][1], nstaged[1], finished && shadow_ray, shadow_entry(slot, hit, k), A.q_shadow[cur], &C.n_shadow[cur],
+        stage_push(A, staged[wib][1], nstaged[1], finished && shadow_ray, shadow_entry(entry & kQueueSlotMask, hit, k), A.q_shadow[cur], &C.n_shadow[cur],
                    lane);
-        q_push(A, A.q_march[cur ^ 1u], &C.n_march[cur ^ 1u], slot, suspend);
+        q_push(A, A.q_march[cur ^ 1u], &C.n_march[cur ^ 1u], entry, suspend);
         if (finished || suspend) phase = MP_EMPTY;
     }
     // The staged remainders.

@@ -82,7 +82,7 @@ PT_DI int path_class(const KScene& S, const Hit& h, bool shadow) {
 // its class.  -1: an index check failed.
 PT_DI int load_staged(const WfArgs& A, const PoolView& v, uint32_t e, bool march, bool result, PathState& ps,
                       float4& contrib, float4* q, uint32_t& local, uint32_t& job, StepResult& r) {
-    const uint32_t slot = result ? (e & kQueueSlotMask) : e;
+    const uint32_t slot = e & kQueueSlotMask;
     if (!pt_check(A, slot, A.pool_size, PT_CHECK_QUEUE_SLOT)) return -1;
     const uint4 w = v.s8[slot];
     job = word_job(w.w);

@@ -31,6 +31,12 @@ struct WfPool {
 // path state).
 constexpr uint32_t kMaxJobRing = 1u << 20;
 
+// March groups: scenes whose SDFs run the same code share one (a batch
+// numbers them, WfJob::group; a MARCH queue entry holds its ray's group above the slot).
+// With several, each iteration sorts its MARCH queue by group, so that a
+// march warp's lanes evaluate one scene's SDFs.
+constexpr int kMarchGroups = 16;
+
 // One render pass of one job: samplesPerFrame samples of every pixel.
 // The table is a ring of job_cap entries: pass number j (counting every pass
 // added since the last reset) lives at jobs[j % job_cap].  Passes [job_lo,
@@ -44,6 +50,7 @@ struct WfJob {
     uint32_t count;       // W*H*spf
     uint32_t finished;    // samples finished (atomic)
     int32_t variant;      // primitive classes of the scene (PT_FEAT_*), for the persistent kernel
+    uint32_t group;       // march group of the scene
     uint32_t local_base;  // pass index of this entry's first sample (a pass split between engines; else 0)
     const KScene* host_scene;  // host copy of *scene (persistent single-pass launches; null: none)
     CamInfo cam;          // camera derived on the device (wf_job_setup)
@@ -69,6 +76,10 @@ struct WfCounters {
     // since the last reset (PT_CHECK_* site, 0: none) and the index it saw.
     uint32_t check_site;
     uint32_t check_index;
+    // With several march groups: the current MARCH queue's entries per group,
+    // and where the next of each goes in the sorted queue.
+    uint32_t group_count[kMarchGroups];
+    uint32_t group_next[kMarchGroups];
 };
 
 // Sites of the index checks of the checked kernel build (PT_DEBUG_CHECKS).
@@ -92,6 +103,7 @@ struct WfArgs {
     uint32_t* q_shade[2];   // primary-ray hits (current, next)
     uint32_t* q_shadow[2];  // shadow-ray results (current, next)
     uint32_t* q_free;
+    uint32_t* q_sorted;  // the current MARCH queue by group (groups > 1)
     WfCounters* counters;
     KTrace trace;  // single-job dispatches only
     uint32_t pool_size;
@@ -99,13 +111,14 @@ struct WfArgs {
     int refill_min;    // idle lanes a march warp gathers before it refills them at once
     int drain_lanes;   // a drained march warp with fewer rays suspends them (0: never)
     int march_inner;   // SDF evaluations per lane between a march warp's refills and queue appends
+    int groups;        // march groups in use (1: the MARCH queue is not sorted)
     int persist_refill;  // ended paths a persistent warp gathers before starting new samples together
 };
 
 // Host side (not seen by the run-time compiled program, pt_jit.cu).
 #if !defined(__CUDACC_RTC__)
 // Bytes of the engine's device buffers for a pool of `pool` slots.
-inline size_t ptk_wavefront_pool_bytes(uint32_t pool) { return (size_t)pool * (14 * 16 + 7 * 4) + 32 * 256; }
+inline size_t ptk_wavefront_pool_bytes(uint32_t pool) { return (size_t)pool * (14 * 16 + 8 * 4) + 32 * 256; }
 
 cudaError_t ptk_wavefront_launch_init(const WfArgs* a, cudaStream_t stream);
 // Writes pass number `index` (camera derived on the device) and publishes
@@ -123,8 +136,9 @@ cudaError_t ptk_wavefront_launch_iteration(const WfArgs* a, bool trace, int grid
 // The built-in march kernel for scenes with SDF plug-ins `kinds` (bit k: kind
 // k; bit 0, slots without a plug-in, is ignored).
 const void* ptk_wavefront_march(uint32_t kinds);
-// Kernels launched per staged iteration (march, shade, gen, bookkeeping).
-constexpr int kWfKernelsPerIteration = 4;
+// Kernels launched per staged iteration: march, shade, gen, bookkeeping, and
+// with several march groups the two that sort the MARCH queue.
+constexpr int kWfKernelsPerIteration = 4, kWfKernelsPerSort = 2;
 // Stages timed by the engine's stage-timing mode.
 enum { PT_STAGE_ISECT = 0, PT_STAGE_MARCH, PT_STAGE_SHADE, PT_STAGE_GEN, PT_STAGE_BOOK, PT_STAGE_COUNT };
 // Persistent mode: one launch of the persistent path kernel over the next

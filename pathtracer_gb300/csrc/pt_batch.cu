@@ -47,6 +47,7 @@ struct BatchScene {
     bool has_sdf = false;
     bool custom = false;        // holds run-time compiled snippets (staged engine only)
     int variant = PT_FEAT_ALL;  // primitive classes present (pt_features.h)
+    uint32_t group = 0;         // march group (its SDFs' code)
     uint32_t passes_in_flight = 0;
 };
 
@@ -132,6 +133,9 @@ struct pt_batch {
     int custom_next = 0;
     JitModule jit;
     bool jit_dirty = false;
+    // March groups (WfJob::group): what the SDF code of each is, the kinds
+    // of built-in plug-ins, or a scene of its own with run-time compiled text.
+    std::vector<uint64_t> groups;
     uint32_t sdf_kinds = 0;  // plug-in kinds of every scene added (bit k: kind k)
     uint32_t jit_kinds = 0;  // the kinds `jit` was compiled for (PT_SDF_KINDS)
     JitModule jit64;  // the FP64 renderer's megakernel for the same snippets (pt_batch_render_fp64), when needed
@@ -484,6 +488,7 @@ int add_scene(pt_batch* b, const pt_ubo* ubo, const pt_sdf_plugin* plugins, int 
     PT_B_TRY(b, cudaSetDevice(b->device));
     KScene* S = new (std::nothrow) KScene;
     if (!S) return bfail(b, PT_ERR_OOM, "pt_batch_add_scene: out of host memory");
+    BatchScene bs;
     std::memset(S, 0, sizeof(KScene));
     std::memcpy(S->numObjects, ubo->numObjects, sizeof(S->numObjects));
     std::memcpy(S->objects, ubo->objects, sizeof(S->objects));
@@ -502,7 +507,12 @@ int add_scene(pt_batch* b, const pt_ubo* ubo, const pt_sdf_plugin* plugins, int 
     S->meta.nplug = nplugins;
     S->meta.custom_base = custom_base;
     pt_derive_cull(S);
-    BatchScene bs;
+    if (n[5] > 0) {
+        const uint64_t code = custom ? (1ull << 32) + b->scenes.size() : kinds;
+        const size_t g = (size_t)(std::find(b->groups.begin(), b->groups.end(), code) - b->groups.begin());
+        if (g == b->groups.size()) b->groups.push_back(code);
+        bs.group = (uint32_t)(g % kMarchGroups);
+    }
     cudaError_t e = cudaMalloc(&bs.d_scene, sizeof(KScene));
     if (e == cudaSuccess) e = cudaMalloc(&bs.d_cie, sizeof(float) * PT_CIE_TABLE_SIZE);
     if (e == cudaSuccess) e = cudaMemcpyAsync(bs.d_scene, S, sizeof(KScene), cudaMemcpyHostToDevice, b->stream);
@@ -664,6 +674,7 @@ int pt_batch_add_pass(pt_batch* b, int scene_id, int target_id, const pt_push* p
     j.colors = p.d_colors;
     j.pc = *push;
     j.variant = sc.variant;
+    j.group = sc.group;
     j.host_scene = e == kPersistent ? sc.h_scene.get() : nullptr;
     const cudaError_t r = E.add_pass_part(j, 0, p.count0, &p.eidx);
     if (r != cudaSuccess) {
@@ -766,6 +777,9 @@ int pt_batch_step(pt_batch* b, int iterations, int* completed, int capacity, int
             PT_B_TRY(b, cudaStreamSynchronize(b->estream[se]));
             b->engine[se].set_march_kernel(staged_march_kernel(b));
         }
+    for (int se : {kStaged, kStaged2})
+        if (b->engine_live[se])
+            b->engine[se].set_groups((int)std::min(std::max(b->groups.size(), (size_t)1), (size_t)kMarchGroups));
     bool busy[kEngines];
     bool any = false;
     for (int e = 0; e < kEngines; e++) {

@@ -36,6 +36,7 @@ size_t layout(uintptr_t base, uint32_t pool, uint32_t max_jobs, WfArgs* a) {
     a->q_shadow[0] = take<uint32_t>(p, pool);
     a->q_shadow[1] = take<uint32_t>(p, pool);
     a->q_free = take<uint32_t>(p, pool);
+    a->q_sorted = take<uint32_t>(p, pool);
     a->counters = take<WfCounters>(p, 1);
     a->jobs = take<WfJob>(p, max_jobs);
     return (size_t)(p - base);
@@ -68,6 +69,7 @@ static cudaError_t common_setup(WfEngine& e, int device, cudaStream_t stream, ui
     e.args.march_budget = march_budget;
     e.args.refill_min = 2;
     e.args.drain_lanes = 24;
+    e.args.groups = 1;
     e.args.march_inner = 6;      // measured best on GB300 (mandelbulb, menger + terrain)
     e.args.persist_refill = 16;  // measured best on GB300 (batch of 64 sphere jobs)
     e.args.trace = KTrace{nullptr, nullptr, nullptr, 0};
@@ -165,6 +167,11 @@ extern const WfKernelSet ptk_wavefront_kernel_set;
 extern const WfKernelSet ptk_wavefront_kernel_set_checked;
 const WfKernelSet* ptk_wavefront_kernels(bool checked) {
     return checked ? &ptk_wavefront_kernel_set_checked : &ptk_wavefront_kernel_set;
+}
+
+void WfEngine::set_groups(int groups) {
+    if (groups != args.groups) drop_graph();
+    args.groups = groups;
 }
 
 void WfEngine::set_march_kernel(const void* kernel) {
@@ -272,11 +279,12 @@ cudaError_t WfEngine::flush_stage_events() {
 }
 
 cudaError_t WfEngine::run(int n, bool trace) {
+    const int per_iteration = kWfKernelsPerIteration + (args.groups > 1 ? kWfKernelsPerSort : 0);
     if (stage_timing && !persistent) {
         for (int i = 0; i < n; i++) {
             if (stage_ev_used == kStageEvRounds) EN_TRY(flush_stage_events());
             EN_TRY(kernels->iteration(&args, trace, grid, stream, &stage_ev[stage_ev_used * 6], march_kernel));
-            kernel_launches += kWfKernelsPerIteration;
+            kernel_launches += (uint64_t)per_iteration;
             stage_ev_used++;
         }
         return flush_stage_events();
@@ -314,12 +322,12 @@ cudaError_t WfEngine::run(int n, bool trace) {
         if (!graph) EN_TRY(build_graph());
         for (; n >= graph_chunk; n -= graph_chunk) {
             EN_TRY(cudaGraphLaunch(graph, stream));
-            kernel_launches += (uint64_t)graph_chunk * kWfKernelsPerIteration;
+            kernel_launches += (uint64_t)(graph_chunk * per_iteration);
         }
     }
     for (int i = 0; i < n; i++) {
         EN_TRY(kernels->iteration(&args, trace, grid, stream, nullptr, march_kernel));
-        kernel_launches += kWfKernelsPerIteration;
+        kernel_launches += (uint64_t)per_iteration;
     }
     return cudaSuccess;
 }

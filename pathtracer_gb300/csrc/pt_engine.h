@@ -159,6 +159,8 @@ struct WfEngine {
     void set_march_budget(int budget);
     // March refill threshold, drain threshold and stage-kernel blocks per SM.
     void set_tuning(int refill_min, int drain_lanes, int blocks_per_sm, int march_inner);
+    // March groups of the scenes rendered (1..kMarchGroups).
+    void set_groups(int groups);
     // Sets march_kernel (null: the built-in kernel).
     void set_march_kernel(const void* kernel);
     // The checked kernel build on or off (the march kernel set by
