@@ -212,10 +212,8 @@ PTM_FN float ptm_scale2(float y, int k) {
     return y * ptm_from_bits((uint32_t)(k + 127) << 23);
 }
 
-PTM_CALL float ptm_expf(float x) {
-    if (x != x) return x;
-    if (x > 88.72283936f) return PTM_INF;
-    if (x < -103.9720840f) return 0.0f;
+/* e^x = y * 2^k: y, and k + PTM_RINT_MAGIC_BITS in *kbits, |x| <= 104. */
+PTM_FN float ptm_exp_reduced(float x, uint32_t* kbits) {
     const float kb = x * PTM_LOG2E + PTM_RINT_MAGIC;
     const float k = kb - PTM_RINT_MAGIC;
     float r = PTM_FMA(-k, PTM_LN2_1, x);
@@ -223,7 +221,17 @@ PTM_CALL float ptm_expf(float x) {
     const float p =
         PTM_FMA(PTM_FMA(PTM_FMA(PTM_FMA(PTM_FMA(PTM_E5, r, PTM_E4), r, PTM_E3), r, PTM_E2), r, PTM_E1), r, PTM_E0);
     const float em1 = PTM_FMA(r * r, p, r); /* e^r - 1 */
-    return ptm_scale2(1.0f + em1, (int)(ptm_bits(kb) - PTM_RINT_MAGIC_BITS));
+    *kbits = ptm_bits(kb);
+    return 1.0f + em1;
+}
+
+PTM_CALL float ptm_expf(float x) {
+    if (x != x) return x;
+    if (x > 88.72283936f) return PTM_INF;
+    if (x < -103.9720840f) return 0.0f;
+    uint32_t kbits;
+    const float y = ptm_exp_reduced(x, &kbits);
+    return ptm_scale2(y, (int)(kbits - PTM_RINT_MAGIC_BITS));
 }
 
 /* log(1+f) for f = m - 1, m in [sqrt(1/2), sqrt(2)]. */
@@ -254,6 +262,27 @@ PTM_FN float ptm_frexp_sqrt2(float x, int* e_out) {
     return m;
 }
 
+/* e * ln2 + log1p_m, for the exponent e and log(m) of a splitting. */
+PTM_FN float ptm_log_join(int e, float log1p_m) {
+    const float ef = ptm_from_bits(PTM_RINT_MAGIC_BITS + (uint32_t)e) - PTM_RINT_MAGIC; /* (float)e */
+    return PTM_FMA(ef, PTM_LN2_1, PTM_FMA(ef, PTM_LN2_2, log1p_m));
+}
+
+/* x positive, normal and finite. */
+PTM_FN int ptm_ordinary(float x) { return (uint32_t)(ptm_bits(x) - 0x00800000u) < 0x7f000000u; }
+
+/* log(x) of an ordinary x: the splitting without its subnormal case. */
+PTM_FN float ptm_log_ordinary(float x) {
+    const uint32_t u = ptm_bits(x);
+    int e = (int)(u >> 23) - 127;
+    float m = ptm_from_bits((u & 0x007fffffu) | 0x3f800000u);
+    if (m > 1.414213538f) {
+        m *= 0.5f;
+        e += 1;
+    }
+    return ptm_log_join(e, ptm_log1p_reduced(m - 1.0f));
+}
+
 PTM_FN float ptm_logf_inline(float x) {
     if (x != x) return x;
     if (x < 0.0f) return PTM_NAN;
@@ -261,9 +290,7 @@ PTM_FN float ptm_logf_inline(float x) {
     if (x == PTM_INF) return x;
     int e;
     const float m = ptm_frexp_sqrt2(x, &e);
-    const float l1p = ptm_log1p_reduced(m - 1.0f);
-    const float ef = ptm_from_bits(PTM_RINT_MAGIC_BITS + (uint32_t)e) - PTM_RINT_MAGIC; /* (float)e */
-    return PTM_FMA(ef, PTM_LN2_1, PTM_FMA(ef, PTM_LN2_2, l1p));
+    return ptm_log_join(e, ptm_log1p_reduced(m - 1.0f));
 }
 
 PTM_CALL float ptm_logf(float x) { return ptm_logf_inline(x); }
@@ -277,7 +304,26 @@ PTM_CALL float ptm_pow_exp_log(float ax, float y) {
     return PTM_FMA(e, perr, e);
 }
 
+/* x^y for an ordinary x and a finite y != 0: the same through one range test
+ * of the exponential's argument (x == 1 gives log 0, hence 1). */
+PTM_CALL float ptm_pow_ordinary(float x, float y) {
+    const float L = ptm_log_ordinary(x);
+    const float p = y * L;
+    const float perr = PTM_FMA(y, L, -p);
+    float e;
+    if (fabsf(p) < 87.0f) {
+        uint32_t kbits;
+        e = ptm_exp_reduced(p, &kbits);
+        e *= ptm_from_bits((kbits - PTM_RINT_MAGIC_BITS + 127u) << 23);
+    } else {
+        e = ptm_expf(p);
+    }
+    return PTM_FMA(e, perr, e);
+}
+
 PTM_FN float ptm_powf(float x, float y) {
+    if (ptm_ordinary(x) && y != 0.0f && fabsf(y) < 16777216.0f && !(fabsf(y) <= 32.0f && floorf(y) == y))
+        return ptm_pow_ordinary(x, y);
     if (y == 0.0f || x == 1.0f) return 1.0f;
     if (x != x || y != y) return PTM_NAN;
     const float ay = fabsf(y);
@@ -318,17 +364,18 @@ PTM_FN float ptm_asin_poly(float x, float z) {
     return PTM_FMA(x * z, A, x);
 }
 
+/* acos and asin evaluate their polynomial once, for x or sqrt((1-|x|)/2): in a
+ * warp whose lanes fall on both sides of 1/2 two calls would run both. */
 PTM_CALL float ptm_acosf(float x) {
     if (x != x) return x;
     const float ax = fabsf(x);
     if (ax > 1.0f) return PTM_NAN;
-    if (ax <= 0.5f) {
-        const float as = ptm_asin_poly(x, x * x);
-        return PTM_PIO2_1 - (as - PTM_PIO2_2);
-    }
-    const float z = (1.0f - ax) * 0.5f;
-    const float s = sqrtf(z);
-    const float as2 = 2.0f * ptm_asin_poly(s, z);
+    const int near0 = ax <= 0.5f;
+    const float z = near0 ? x * x : (1.0f - ax) * 0.5f;
+    const float s = near0 ? x : sqrtf(z);
+    const float as = ptm_asin_poly(s, z);
+    if (near0) return PTM_PIO2_1 - (as - PTM_PIO2_2);
+    const float as2 = 2.0f * as;
     if (x > 0.0f) return as2;
     return PTM_PI_1 - (as2 - PTM_PI_2);
 }
@@ -338,14 +385,11 @@ PTM_CALL float ptm_asinf(float x) {
     if (x != x) return x;
     const float ax = fabsf(x);
     if (ax > 1.0f) return PTM_NAN;
-    float r;
-    if (ax <= 0.5f) {
-        r = ptm_asin_poly(ax, ax * ax);
-    } else {
-        const float z = (1.0f - ax) * 0.5f;
-        const float s = sqrtf(z);
-        r = PTM_PIO2_1 - (2.0f * ptm_asin_poly(s, z) - PTM_PIO2_2);
-    }
+    const int near0 = ax <= 0.5f;
+    const float z = near0 ? ax * ax : (1.0f - ax) * 0.5f;
+    const float s = near0 ? ax : sqrtf(z);
+    const float as = ptm_asin_poly(s, z);
+    const float r = near0 ? as : PTM_PIO2_1 - (2.0f * as - PTM_PIO2_2);
     return (ptm_bits(x) >> 31) ? -r : r;
 }
 
@@ -367,13 +411,8 @@ PTM_FN float ptm_atan_poly(float r) {
 PTM_CALL float ptm_atanf(float x) {
     if (x != x) return x;
     const float a = fabsf(x);
-    float r;
-    if (a > 1.0f) {
-        const float p = ptm_atan_poly(1.0f / a);
-        r = PTM_PIO2_1 - (p - PTM_PIO2_2);
-    } else {
-        r = ptm_atan_poly(a);
-    }
+    const float p = ptm_atan_poly(a > 1.0f ? 1.0f / a : a);
+    const float r = a > 1.0f ? PTM_PIO2_1 - (p - PTM_PIO2_2) : p;
     return (ptm_bits(x) >> 31) ? -r : r;
 }
 
@@ -391,7 +430,7 @@ PTM_CALL float ptm_atan2f(float y, float x) {
         r = xneg ? PTM_PI_1 : 0.0f;
     } else {
         const int swap = ay > ax;
-        const float t = swap ? ax / ay : ay / ax;
+        const float t = (swap ? ax : ay) / (swap ? ay : ax); /* one division for both cases */
         const float p = ptm_atan_poly(t);
         r = swap ? PTM_PIO2_1 - (p - PTM_PIO2_2) : p;
         if (xneg) r = PTM_PI_1 - (r - PTM_PI_2);

@@ -285,3 +285,74 @@ def test_export_forms_are_the_plain_chain(tmp_path, first, step):
     fn = ctypes.CDLL(str(lib)).export_differs
     fn.restype, fn.argtypes = ctypes.c_long, [ctypes.c_uint32, ctypes.c_uint32]
     assert fn(first, step) == 0
+
+
+INVERSE_C = r"""
+#include "pt_mathf.h"
+/* the forms with a branch per case: two polynomials, two divisions, a check per special argument of pow */
+static float acos_plain(float x) {
+    if (x != x) return x;
+    const float ax = fabsf(x);
+    if (ax > 1.0f) return PTM_NAN;
+    if (ax <= 0.5f) return PTM_PIO2_1 - (ptm_asin_poly(x, x * x) - PTM_PIO2_2);
+    const float z = (1.0f - ax) * 0.5f, as2 = 2.0f * ptm_asin_poly(sqrtf(z), z);
+    return x > 0.0f ? as2 : PTM_PI_1 - (as2 - PTM_PI_2);
+}
+static float asin_plain(float x) {
+    if (x != x) return x;
+    const float ax = fabsf(x), z = (1.0f - ax) * 0.5f;
+    if (ax > 1.0f) return PTM_NAN;
+    const float r = ax <= 0.5f ? ptm_asin_poly(ax, ax * ax) : PTM_PIO2_1 - (2.0f * ptm_asin_poly(sqrtf(z), z) - PTM_PIO2_2);
+    return (ptm_bits(x) >> 31) ? -r : r;
+}
+static float atan_plain(float x) {
+    if (x != x) return x;
+    const float a = fabsf(x);
+    const float r = a > 1.0f ? PTM_PIO2_1 - (ptm_atan_poly(1.0f / a) - PTM_PIO2_2) : ptm_atan_poly(a);
+    return (ptm_bits(x) >> 31) ? -r : r;
+}
+static float pow_plain(float x, float y) {  /* y finite, not 0 and not an integer of magnitude <= 32 */
+    if (x == 1.0f) return 1.0f;
+    if (x != x) return PTM_NAN;
+    const float ax = fabsf(x), ay = fabsf(y);
+    const int odd = floorf(ay) == ay && ay < 16777216.0f && (int)(ay - 2.0f * floorf(ay * 0.5f)) == 1;
+    const int neg = x < 0.0f && odd;
+    if (x < 0.0f && floorf(ay) != ay) return PTM_NAN;
+    float r;
+    if (ax == 0.0f || ax == PTM_INF) r = ((ax == 0.0f) == (y > 0.0f)) ? 0.0f : PTM_INF;
+    else r = ptm_pow_exp_log(ax, y);
+    return neg ? -r : r;
+}
+static int ne(float a, float b) { return ptm_bits(a) != ptm_bits(b) && !(a != a && b != b); }
+long inverse_differ(uint32_t first, uint32_t step) {
+    static const float ys[] = {1.0f / 2.4f, 8.23f, -2.5f, 0.3333333f, 33.0f, 100.5f, -41.0f, 1e7f};
+    long bad = 0;
+    uint64_t u;
+    unsigned k;
+    for (u = first; u < (1ull << 32); u += step) {
+        const float x = ptm_from_bits((uint32_t)u), y = ptm_from_bits((uint32_t)u * 2654435761u + 977u);
+        bad += ne(ptm_acosf(x), acos_plain(x)) + ne(ptm_asinf(x), asin_plain(x)) + ne(ptm_atanf(x), atan_plain(x));
+        for (k = 0; k < sizeof ys / sizeof ys[0]; k++) bad += ne(ptm_powf(x, ys[k]), pow_plain(x, ys[k]));
+        if (x == x && y == y && fabsf(x) < 1e38f && fabsf(y) < 1e38f && x != 0.0f) {  /* the general case of atan2 */
+            const float ax = fabsf(y), ay = fabsf(x), t = ay > ax ? ax / ay : ay / ax, p = ptm_atan_poly(t);
+            float r = ay > ax ? PTM_PIO2_1 - (p - PTM_PIO2_2) : p;
+            if (ptm_bits(y) >> 31) r = PTM_PI_1 - (r - PTM_PI_2);
+            bad += ne(ptm_atan2f(x, y), (ptm_bits(x) >> 31) ? -r : r);
+        }
+    }
+    return bad;
+}
+"""
+
+
+@pytest.mark.parametrize("first", [0, 7])
+def test_inverse_functions_and_pow_are_the_plain_forms(tmp_path, first):
+    import ctypes
+
+    src, lib = tmp_path / "i.c", tmp_path / "i.so"
+    src.write_text(INVERSE_C)
+    subprocess.run([os.environ.get("CC", "gcc"), "-O2", "-std=c11", "-ffp-contract=off", "-fPIC", "-shared",
+                    "-I" + os.path.join(ROOT, "include"), "-o", str(lib), str(src), "-lm"], check=True)
+    fn = ctypes.CDLL(str(lib)).inverse_differ
+    fn.restype, fn.argtypes = ctypes.c_long, [ctypes.c_uint32, ctypes.c_uint32]
+    assert fn(first, 4099) == 0
