@@ -28,6 +28,7 @@ struct pt_ctx {
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
+    cudaEvent_t busy = nullptr;    // after the last dispatch on an engine of the context (pt_set_stream)
     KParams* params = nullptr;  // host image of the launch parameters
     bool has_scene = false;
     float* d_cie = nullptr;
@@ -146,6 +147,7 @@ int pt_create(pt_ctx** out, int device) {
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->done, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->busy, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_cie, sizeof(float) * PT_CIE_TABLE_SIZE);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_rot, sizeof(float) * 9 * PT_MAX_SCENE_OBJECTS);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_scene, sizeof(KScene));
@@ -191,6 +193,7 @@ int pt_destroy(pt_ctx* ctx) {
     for (auto& cache : ctx->jit)
         for (JitModule& m : cache) pt_jit_unload(m);
     if (ctx->done) cudaEventDestroy(ctx->done);
+    if (ctx->busy) cudaEventDestroy(ctx->busy);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx->params;
     delete ctx;
@@ -673,9 +676,20 @@ int pt_set_stream(pt_ctx* ctx, void* stream) {
     const cudaStream_t s = stream ? (cudaStream_t)stream : ctx->own_stream;
     if (s != ctx->stream) {
         // The scene's device copy, the colour buffer and the engines belong to
-        // the last dispatch until it is done.
+        // the last dispatch that used them until it is done.
         PT_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-        PT_CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->done, 0));
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        PT_CUDA_TRY(ctx, cudaStreamIsCapturing(s, &capture));
+        if (capture == cudaStreamCaptureStatusNone) {
+            PT_CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->busy, 0));
+        } else {
+            // a captured wait would bind the capture to work outside it: wait here
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            PT_CUDA_TRY(ctx, cudaThreadExchangeStreamCaptureMode(&mode));
+            const cudaError_t e = cudaEventSynchronize(ctx->busy);
+            PT_CUDA_TRY(ctx, cudaThreadExchangeStreamCaptureMode(&mode));
+            PT_CUDA_TRY(ctx, e);
+        }
     }
     ctx->stream = s;
     return PT_OK;
@@ -707,6 +721,15 @@ const char* pt_last_error(pt_ctx* ctx) {
 }
 
 }  // extern "C"
+
+// Marks the end of a dispatch that used the context's engines.  Not inside a
+// stream capture: other streams cannot wait for an event of one.
+static cudaError_t record_busy(pt_ctx* ctx) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(ctx->stream, &capture);
+    if (e != cudaSuccess || capture != cudaStreamCaptureStatusNone) return e;
+    return cudaEventRecord(ctx->busy, ctx->stream);
+}
 
 // A dispatch of a scene without SDFs, or of few samples: one pass on the
 // persistent kernel, in one launch, then the resolve.  Nothing is read back, so the call returns
@@ -758,6 +781,7 @@ static int dispatch_persistent(pt_ctx* ctx, const pt_push* push) {
     ctx->last_iterations = 1;
     ctx->last_launches = E.kernel_launches - launches0;
     PT_CUDA_TRY(ctx, cudaEventRecord(ctx->done, ctx->stream));
+    PT_CUDA_TRY(ctx, record_busy(ctx));
     return PT_OK;
 }
 
@@ -882,6 +906,7 @@ static int dispatch_wavefront(pt_ctx* ctx, const pt_push* push) {
         if (*slot[e]) launches1 += (*slot[e])->kernel_launches;
     ctx->last_launches = launches1 - launches0;
     PT_CUDA_TRY(ctx, cudaEventRecord(ctx->done, ctx->stream));
+    PT_CUDA_TRY(ctx, record_busy(ctx));
     return PT_OK;
 }
 
