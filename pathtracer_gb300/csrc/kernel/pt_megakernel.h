@@ -22,7 +22,10 @@ cudaError_t ptk_launch_megakernel(const KParams* params, bool trace, cudaStream_
 // One dispatch of the FP64 reference renderer (pt_fp64.cu): the same paths
 // in double precision, adding exposed colour sums and sample counts to
 // params->sums (4 doubles per pixel).
-cudaError_t ptk_launch_fp64(const KParams* params, bool trace, cudaStream_t stream);
+// scratch: ptk_fp64_scratch(&params->pc) bytes of device memory that are the
+// dispatch's until it is done; null: rendered without (slower, same bits).
+cudaError_t ptk_launch_fp64(const KParams* params, bool trace, void* scratch, int sms, cudaStream_t stream);
+size_t ptk_fp64_scratch(const pt_push* pc);  // 0: the dispatch takes none
 // The analytic-scene variants (PT_FEAT_* 0, BOX, ANALYTIC), from their own
 // translation unit.
 cudaError_t ptk_launch_megakernel_analytic(const KParams* params, int variant, dim3 grid, dim3 block,

@@ -62,6 +62,8 @@ struct pt_ctx {
     float4* d_colors = nullptr;    // per-sample colours of the current dispatch
     uint8_t* d_rgb = nullptr;      // pt_read_rgb8 staging (W*H*3 bytes)
     size_t rgb_bytes = 0;
+    void* d_fp64 = nullptr;        // pt_render_fp64's sample colours (ptk_fp64_scratch: 48 MB at most)
+    size_t fp64_bytes = 0;
     size_t colors_bytes = 0;
     uint32_t last_iterations = 0;
     uint64_t last_launches = 0;    // kernels the last pt_dispatch launched
@@ -126,6 +128,8 @@ constexpr uint64_t kSmallDispatch = 1ull << 18;
 
 static int dispatch_wavefront(pt_ctx* ctx, const pt_push* push);
 static int dispatch_persistent(pt_ctx* ctx, const pt_push* push);
+static cudaError_t record_busy(pt_ctx* ctx);
+static cudaError_t fp64_scratch(pt_ctx* ctx, const pt_push* push, void** scratch, int* sms);
 static int dispatch_jit(pt_ctx* ctx, bool trace);
 static int ensure_jit(pt_ctx* ctx, JitKind kind);
 cudaError_t ptk_export_rgb8(const void* d_accum, int width, int height, int tonemap, void* d_rgb, cudaStream_t stream);
@@ -190,6 +194,7 @@ int pt_destroy(pt_ctx* ctx) {
         if (s) cudaStreamDestroy(s);
     if (ctx->d_colors) cudaFree(ctx->d_colors);
     if (ctx->d_rgb) cudaFree(ctx->d_rgb);
+    if (ctx->d_fp64) cudaFree(ctx->d_fp64);
     for (auto& cache : ctx->jit)
         for (JitModule& m : cache) pt_jit_unload(m);
     if (ctx->done) cudaEventDestroy(ctx->done);
@@ -419,12 +424,19 @@ int pt_render_fp64(pt_ctx* ctx, const pt_push* push, double* d_sums) {
     P.cie = ctx->d_cie;
     P.trace = ctx->trace;
     const bool trace = ctx->trace.events || ctx->trace.nevents || ctx->trace.colors;
-    const cudaError_t e =
-        ctx->custom.empty() ? ptk_launch_fp64(&P, trace, ctx->stream)
-                            : pt_jit_launch(ctx->jit[kJitFp64][(size_t)ctx->jit_cur[kJitFp64]], &P, trace, ctx->stream);
+    cudaError_t e;
+    if (ctx->custom.empty()) {
+        void* scratch = nullptr;
+        int sms = 0;
+        e = fp64_scratch(ctx, push, &scratch, &sms);
+        if (e == cudaSuccess) e = ptk_launch_fp64(&P, trace, scratch, sms, ctx->stream);
+    } else {
+        e = pt_jit_launch(ctx->jit[kJitFp64][(size_t)ctx->jit_cur[kJitFp64]], &P, trace, ctx->stream);
+    }
     P.sums = nullptr;
     PT_CUDA_TRY(ctx, e);
     PT_CUDA_TRY(ctx, cudaEventRecord(ctx->done, ctx->stream));
+    PT_CUDA_TRY(ctx, record_busy(ctx));
     return PT_OK;
 }
 
@@ -729,6 +741,32 @@ static cudaError_t record_busy(pt_ctx* ctx) {
     const cudaError_t e = cudaStreamIsCapturing(ctx->stream, &capture);
     if (e != cudaSuccess || capture != cudaStreamCaptureStatusNone) return e;
     return cudaEventRecord(ctx->busy, ctx->stream);
+}
+
+// The FP64 renderer's scratch; null for a dispatch that takes none, without
+// memory for it, or captured (a graph would keep the pointer).
+static cudaError_t fp64_scratch(pt_ctx* ctx, const pt_push* push, void** scratch, int* sms) {
+    *scratch = nullptr;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(ctx->stream, &capture);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    const size_t need = ptk_fp64_scratch(push);
+    if (e != cudaSuccess || capture != cudaStreamCaptureStatusNone || need == 0) return e;
+    if (ctx->fp64_bytes < need) {
+        e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) return e;
+        if (ctx->d_fp64) cudaFree(ctx->d_fp64);
+        ctx->d_fp64 = nullptr;
+        ctx->fp64_bytes = 0;
+        if (cudaMalloc(&ctx->d_fp64, need) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->d_fp64 = nullptr;
+            return cudaSuccess;
+        }
+        ctx->fp64_bytes = need;
+    }
+    *scratch = ctx->d_fp64;
+    return cudaSuccess;
 }
 
 // A dispatch of a scene without SDFs, or of few samples: one pass on the

@@ -917,7 +917,20 @@ int pt_batch_render_fp64(pt_batch* b, int scene_id, int target_id, const pt_push
         P->pc = *push;
         P->cie = sc.d_cie;
         P->sums = t.d_sum;
-        e = sc.custom ? pt_jit_launch(b->jit64, P, false, b->stream) : ptk_launch_fp64(P, false, b->stream);
+        if (sc.custom) {
+            e = pt_jit_launch(b->jit64, P, false, b->stream);
+        } else {
+            void* scratch = nullptr;  // without memory for it: rendered without
+            int sms = 0;
+            const size_t need = ptk_fp64_scratch(push);
+            if (need > 0 && cudaMallocFromPoolAsync(&scratch, need, b->mempool, b->stream) != cudaSuccess) {
+                cudaGetLastError();
+                scratch = nullptr;
+            }
+            e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
+            if (e == cudaSuccess) e = ptk_launch_fp64(P, false, scratch, sms, b->stream);
+            if (scratch) cudaFreeAsync(scratch, b->stream);
+        }
         b->kernel_launches += 1;
     }
     delete P;
