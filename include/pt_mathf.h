@@ -169,10 +169,13 @@ PTM_FN ptm_sc ptm_sincos_small(float x) {
     return ptm_sincos_quadrant(ptm_sincos_reduce(x, kb - PTM_RINT_MAGIC), ptm_bits(kb));
 }
 
-/* sin and cos of x together. */
+/* sin and cos of x together.  The common form is computed before the test:
+ * straight-line code is shared by every sine and cosine of one x that is
+ * inlined, code under a branch of each is not. */
 PTM_FN ptm_sc ptm_sincos_inline(float x) {
-    if (!(fabsf(x * PTM_2_OVER_PI) < 4194304.0f)) return ptm_sincos_large(x);
-    return ptm_sincos_small(x);
+    ptm_sc r = ptm_sincos_small(x);
+    if (!(fabsf(x * PTM_2_OVER_PI) < 4194304.0f)) r = ptm_sincos_large(x);
+    return r;
 }
 
 PTM_CALL ptm_sc ptm_sincos_v(float x) { return ptm_sincos_inline(x); }
@@ -304,10 +307,9 @@ PTM_CALL float ptm_pow_exp_log(float ax, float y) {
     return PTM_FMA(e, perr, e);
 }
 
-/* x^y for an ordinary x and a finite y != 0: the same through one range test
- * of the exponential's argument (x == 1 gives log 0, hence 1). */
-PTM_CALL float ptm_pow_ordinary(float x, float y) {
-    const float L = ptm_log_ordinary(x);
+/* x^y from L = log(x) of an ordinary x and a finite y != 0: the same through
+ * one range test of the exponential's argument (x == 1 gives log 0, hence 1). */
+PTM_FN float ptm_pow_of_log(float L, float y) {
     const float p = y * L;
     const float perr = PTM_FMA(y, L, -p);
     float e;
@@ -321,9 +323,20 @@ PTM_CALL float ptm_pow_ordinary(float x, float y) {
     return PTM_FMA(e, perr, e);
 }
 
+PTM_CALL float ptm_pow_ordinary(float x, float y) { return ptm_pow_of_log(ptm_log_ordinary(x), y); }
+
 PTM_FN float ptm_powf(float x, float y) {
-    if (ptm_ordinary(x) && y != 0.0f && fabsf(y) < 16777216.0f && !(fabsf(y) <= 32.0f && floorf(y) == y))
+#if !defined(PTM_OUTLINE)
+    /* before the test, so that inlined powers of one x share it (ptm_sincos_inline) */
+    const float L = ptm_log_ordinary(x);
+#endif
+    if (ptm_ordinary(x) && y != 0.0f && fabsf(y) < 16777216.0f && !(fabsf(y) <= 32.0f && floorf(y) == y)) {
+#if defined(PTM_OUTLINE)
         return ptm_pow_ordinary(x, y);
+#else
+        return ptm_pow_of_log(L, y);
+#endif
+    }
     if (y == 0.0f || x == 1.0f) return 1.0f;
     if (x != x || y != y) return PTM_NAN;
     const float ay = fabsf(y);
