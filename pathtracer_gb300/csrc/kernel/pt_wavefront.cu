@@ -31,6 +31,7 @@
 // before use; pt_check in pt_march.cuh) and its launch functions renamed by
 // PTK_WF; the engine picks either set (ptk_wavefront_kernels).
 #define PTM_OUTLINE
+#define PT_UNROLL_MENGER
 #include <cuda_runtime.h>
 
 #ifndef PTK_WF

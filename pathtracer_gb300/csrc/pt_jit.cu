@@ -72,6 +72,7 @@ std::string pt_jit_program(const std::vector<JitSlot>& slots, JitKind kind) {
         s += "#include \"pt_megakernel_body.cuh\"\n";
         return s;
     }
+    if (kind == kJitMarch) s += "#define PT_UNROLL_MENGER 1\n";
     s += "#include \"pt_glsl_shim.h\"\n";
     for (const JitSlot& j : slots) s += j.code + "\n";
     s += "static __device__ __forceinline__ float pt_user_sdf(int slot, float3 p) {\n  switch (slot) {\n";
