@@ -239,14 +239,17 @@ int pt_render_fp64(pt_ctx* ctx, const pt_push* push, double* d_sums);
  *   PT_ENGINE_WAVEFRONT (default): every sample is a work item in a pool of
  *     path slots in device memory; compacted ray queues per stage and a
  *     persistent SDF-march kernel; per-sample XYZ summed per pixel in sample
- *     order at the end.  Allocates its scratch on first use; pt_dispatch
- *     returns once the dispatch is resolved on the stream. */
+ *     order at the end.  Allocates its scratch on first use.  Dispatches of
+ *     scenes without SDFs, and of up to 2^18 samples of built-in SDFs, run on
+ *     the persistent kernel instead, unless a staged knob, a trace, stage
+ *     times, checks or a drain limit is set.  pt_dispatch may return with work
+ *     queued on the stream; pt_set_stream orders the new stream after it. */
 #define PT_ENGINE_MEGAKERNEL 0
 #define PT_ENGINE_WAVEFRONT 1
 int pt_set_engine(pt_ctx* ctx, int engine);
 int pt_get_engine(pt_ctx* ctx);
 /* Path slots of the wavefront pool (default 2^22: a deeper pool keeps more
- * rays to refill march lanes from; 252 B each, plus 16 B per sample of the
+ * rays to refill march lanes from; 256 B each, plus 16 B per sample of the
  * dispatch for the sample colours; a dispatch uses at most its own sample
  * count of slots). */
 int pt_set_wavefront_pool(pt_ctx* ctx, uint32_t slots);
