@@ -161,13 +161,13 @@ extern "C" int pt_jit_check(const char* const* sources, int n, int sm, char* log
         std::vector<char> cubin;
         std::string lowered[kJitMaxKernels];
         // what a context compiles for a scene of these snippets: its march
-        // kernel holds no built-in plug-in, and for one snippet the
-        // megakernel and march kernel evaluate it without the loop over the
+        // kernel, and its megakernel for several, hold no built-in plug-in,
+        // and for one snippet both evaluate it without the loop over the
         // SDF set
         const bool fp32 = k == kJitMegakernel || k == kJitMarch;
         const std::string head =
             std::string(fp32 && n == 1 ? "#define PT_ONE_SDF 1\n" : "") +
-            (k == kJitMarch ? "#define PT_SDF_KINDS " + std::to_string(1u << PT_SDF_CUSTOM) + "u\n" : "");
+            (k == kJitMarch || (k == kJitMegakernel && n > 1) ? "#define PT_SDF_KINDS " + std::to_string(1u << PT_SDF_CUSTOM) + "u\n" : "");
         rc = pt_jit_compile_for(sm, head + pt_jit_program(slots, (JitKind)k), (JitKind)k, cubin, lowered, msg);
         all += msg;
     }
