@@ -305,6 +305,12 @@ size_t ptk_fp64_scratch(const pt_push* pc) {
     return 256 + 24 * (size_t)(total < kFp64Span ? total : kFp64Span);
 }
 
+uint64_t ptk_fp64_kernels(const pt_push* pc, const void* scratch) {
+    if (!scratch) return 1;
+    const uint64_t per = kFp64Span / (uint64_t)pc->samplesPerFrame;
+    return 2 * (((uint64_t)pc->resolution[0] * (uint64_t)pc->resolution[1] + per - 1) / per);
+}
+
 cudaError_t ptk_launch_fp64(const KParams* params, bool trace, void* scratch, int sms, cudaStream_t stream) {
     const int W = params->pc.resolution[0], H = params->pc.resolution[1];
     const uint64_t pixels = (uint64_t)W * (uint64_t)H;

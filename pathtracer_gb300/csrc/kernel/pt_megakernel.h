@@ -26,6 +26,7 @@ cudaError_t ptk_launch_megakernel(const KParams* params, bool trace, cudaStream_
 // dispatch's until it is done; null: rendered without (slower, same bits).
 cudaError_t ptk_launch_fp64(const KParams* params, bool trace, void* scratch, int sms, cudaStream_t stream);
 size_t ptk_fp64_scratch(const pt_push* pc);  // 0: the dispatch takes none
+uint64_t ptk_fp64_kernels(const pt_push* pc, const void* scratch);  // kernels that a dispatch without trace launches
 // The analytic-scene variants (PT_FEAT_* 0, BOX, ANALYTIC), from their own
 // translation unit.
 cudaError_t ptk_launch_megakernel_analytic(const KParams* params, int variant, dim3 grid, dim3 block,

@@ -919,6 +919,7 @@ int pt_batch_render_fp64(pt_batch* b, int scene_id, int target_id, const pt_push
         P->sums = t.d_sum;
         if (sc.custom) {
             e = pt_jit_launch(b->jit64, P, false, b->stream);
+            b->kernel_launches += 1;
         } else {
             void* scratch = nullptr;  // without memory for it: rendered without
             int sms = 0;
@@ -930,8 +931,8 @@ int pt_batch_render_fp64(pt_batch* b, int scene_id, int target_id, const pt_push
             e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
             if (e == cudaSuccess) e = ptk_launch_fp64(P, false, scratch, sms, b->stream);
             if (scratch) cudaFreeAsync(scratch, b->stream);
+            b->kernel_launches += ptk_fp64_kernels(push, scratch);
         }
-        b->kernel_launches += 1;
     }
     delete P;
     if (e != cudaSuccess) return bcuda(b, e, "pt_batch_render_fp64");
