@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include "pt_megakernel_body.cuh"
+#include "pt_share.h"
 
 namespace {
 
@@ -287,7 +288,7 @@ cudaError_t launch_paths(const KParams* params, int sms, uint64_t pixels, unsign
         // have full lists too; the samples shared by all warps, eight or more each.
         const int blocks = sms * (span.total < kFp64Wide ? 1 : per_sm);
         const uint32_t warps = (uint32_t)(blocks * kFp64Warps), share = (span.total + warps - 1) / warps;
-        span.slots = share < 8 ? 8 : share < (uint32_t)kFp64Slots ? (int)share : kFp64Slots;
+        span.slots = warp_slots(share, 8, 1, kFp64Slots);
         e = cudaMemsetAsync(span.cursor, 0, sizeof(uint32_t), stream);
         if (e != cudaSuccess) return e;
         fp64_paths<FEAT><<<blocks, kFp64Threads, sizeof(Fp64Shared), stream>>>(*params, span);

@@ -14,6 +14,7 @@
 
 #include "pt_march.cuh"
 #include "pt_ring.cuh"
+#include "pt_share.h"
 #include "pt_wavefront.h"
 
 namespace {
@@ -47,6 +48,7 @@ constexpr int kPersistWarps = kPersistThreads / 32;
 constexpr int kPersistQuads = 7;
 // The classes of steps, and what a path on the PC_END list still needs.
 enum PathClass { PC_SHADOW = 0, PC_DIFFUSE, PC_SPECULAR, PC_END, PC_COUNT };
+static_assert(kPersistSlots <= 256, "a list entry holds its slot in 8 bits");
 enum PathEnd { PE_HIT = 0, PE_COLOUR = 1, PE_START = 2 };  // shade an emitter or miss; write the colour; start
 struct PersistShared {
     float4 state[kPersistWarps][kPersistSlots * kPersistQuads];
@@ -164,7 +166,7 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
     const uint64_t share = (end - (POOL ? 0 : C.pk_begin)) / ((uint64_t)gridDim.x * kPersistWarps);
     // A staged engine's last paths are spread over every warp: their time is
     // the longest path's, and a warp steps as long as its longest march.
-    const int slots = POOL ? min(kPersistSlots, (int)share + 1) : share >= (uint64_t)kPersistSlots ? kPersistSlots : (share < 32 ? 32 : (int)((share + 31) / 32 * 32));
+    const int slots = POOL ? warp_slots(share + 1, 1, 1, kPersistSlots) : warp_slots(share, 32, 32, kPersistSlots);
     const uint32_t chunk = POOL ? min(32u, (uint32_t)share + 1) : share >= 8 * kPersistChunk ? kPersistChunk : (share < 128 ? 32u : (uint32_t)(share / 128 * 32));
     int count[PC_COUNT] = {0, 0, 0, 0};  // warp-uniform: the lists' lengths
     for (int i = lane; i < slots; i += 32) sh.list[warp][PC_END][i] = (uint16_t)(i | (PE_START << 8));
@@ -202,6 +204,7 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
             const uint32_t e = sh.list[warp][cls][from + lane];
             slot = e & 0xffu;
             ends = (int)(e >> 8);
+            live = pt_check(A, slot, (uint32_t)slots, PT_CHECK_WARP_SLOT);
         }
         __syncwarp();
         float4* const q = st + slot * kPersistQuads;
@@ -357,7 +360,9 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
 #pragma unroll
         for (int c = 0; c < PC_COUNT; c++) {
             const unsigned m = __ballot_sync(0xffffffffu, next == c);
-            if (next == c) sh.list[warp][c][count[c] + __popc(m & lt)] = (uint16_t)(slot | (uint32_t)(next_end << 8));
+            const uint32_t at = (uint32_t)(count[c] + __popc(m & lt));
+            if (next == c && pt_check(A, at, kPersistSlots, PT_CHECK_WARP_LIST))
+                sh.list[warp][c][at] = (uint16_t)(slot | (uint32_t)(next_end << 8));
             count[c] += __popc(m);
         }
         __syncwarp();

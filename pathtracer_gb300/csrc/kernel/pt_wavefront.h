@@ -91,6 +91,8 @@ enum {
     PT_CHECK_JOB = 4,           // a pass index outside the job ring
     PT_CHECK_SAMPLE = 5,        // a sample index outside its pass (colour buffer)
     PT_CHECK_QUEUE_COUNT = 6,   // a queue or free-list length above the pool size after an iteration
+    PT_CHECK_WARP_SLOT = 7,     // persistent kernel: a slot outside a warp's arrays
+    PT_CHECK_WARP_LIST = 8,     // persistent kernel: an append past a warp's list
 };
 
 // Everything here is fixed between resets, so a captured chain of iterations

@@ -65,6 +65,8 @@ inline const char* pt_check_site_name(uint32_t site) {
         case PT_CHECK_JOB: return "pass index outside the job ring";
         case PT_CHECK_SAMPLE: return "sample index outside its pass";
         case PT_CHECK_QUEUE_COUNT: return "queue length above the pool size";
+        case PT_CHECK_WARP_SLOT: return "path slot outside the warp's arrays";
+        case PT_CHECK_WARP_LIST: return "append past a warp's list";
         default: return "unknown site";
     }
 }
