@@ -235,7 +235,7 @@ int pt_render_fp64(pt_ctx* ctx, const pt_push* push, double* d_sums);
 /* Engines behind pt_dispatch; both compute the reference's per-sample
  * arithmetic bit for bit and differ only in scheduling.
  *   PT_ENGINE_MEGAKERNEL: one thread per pixel, samples in order (the plain
- *     method).  Asynchronous.
+ *     method).  Asynchronous, and may be captured into a graph.
  *   PT_ENGINE_WAVEFRONT (default): every sample is a work item in a pool of
  *     path slots in device memory; compacted ray queues per stage and a
  *     persistent SDF-march kernel; per-sample XYZ summed per pixel in sample
@@ -243,7 +243,9 @@ int pt_render_fp64(pt_ctx* ctx, const pt_push* push, double* d_sums);
  *     scenes without SDFs, and of up to 2^18 samples of built-in SDFs, run on
  *     the persistent kernel instead, unless a staged knob, a trace, stage
  *     times, checks or a drain limit is set.  pt_dispatch may return with work
- *     queued on the stream; pt_set_stream orders the new stream after it. */
+ *     queued on the stream; pt_set_stream orders the new stream after it.
+ *     Refused (PT_ERR_CUDA) in a stream capture: a graph would keep buffers
+ *     that later dispatches free or use. */
 #define PT_ENGINE_MEGAKERNEL 0
 #define PT_ENGINE_WAVEFRONT 1
 int pt_set_engine(pt_ctx* ctx, int engine);

@@ -377,14 +377,23 @@ int pt_dispatch(pt_ctx* ctx, const pt_push* push) {
     P.cie = ctx->d_cie;
     P.trace = ctx->trace;
     const bool trace = ctx->trace.events || ctx->trace.nevents || ctx->trace.colors;
+    const bool wavefront = ctx->engine == PT_ENGINE_WAVEFRONT && push->pathLength > 0;
+    if (wavefront) {
+        // A graph would keep the engine's buffers, which a larger dispatch
+        // frees and every other dispatch uses too.
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        PT_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &capture));
+        if (capture != cudaStreamCaptureStatusNone)
+            return cuda_fail(ctx, cudaErrorStreamCaptureUnsupported,
+                             "pt_dispatch on PT_ENGINE_WAVEFRONT (PT_ENGINE_MEGAKERNEL can be captured)");
+    }
     if (!ctx->custom.empty()) {
-        const bool staged = ctx->engine == PT_ENGINE_WAVEFRONT && push->pathLength > 0;
-        const int rc = ensure_jit(ctx, staged ? kJitMarch : kJitMegakernel);
+        const int rc = ensure_jit(ctx, wavefront ? kJitMarch : kJitMegakernel);
         if (rc != PT_OK) return rc;
         ctx->last_launches = 1;
-        if (!staged) return dispatch_jit(ctx, trace);
+        if (!wavefront) return dispatch_jit(ctx, trace);
     }
-    if (ctx->engine == PT_ENGINE_WAVEFRONT && push->pathLength > 0) {
+    if (wavefront) {
         // A scene without SDFs has nothing for the staged kernels to sort:
         // its paths stay on chip in the persistent kernel (dispatch_persistent).
         // Whatever asks for the staged kernels themselves gets them: traces,
