@@ -475,8 +475,9 @@ typedef struct pt_batch_info {
     uint64_t kernel_launches; /* kernels the batch has launched (graph replays counted per kernel) */
 } pt_batch_info;
 
-/* pool_slots >= 1024 paths in flight in each staged engine; max_passes
- * passes of each engine in flight at once. */
+/* pool_slots >= 1024 paths in flight in each staged engine (more than 2^28 are
+ * taken as 2^28: the same images); max_passes passes of each engine in flight
+ * at once. */
 int pt_batch_create(pt_batch** out, int device, uint32_t pool_slots, uint32_t max_passes);
 int pt_batch_destroy(pt_batch* batch);
 const char* pt_batch_last_error(pt_batch* batch);

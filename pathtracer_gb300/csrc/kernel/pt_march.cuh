@@ -103,11 +103,11 @@ struct PoolView {
     PairField<float4> s9, h0, h1, m0, m1;
 };
 
-// An entry of the shadow queues: the slot (pools have at most 2^28) and what
+// An entry of the shadow queues: the slot and what
 // the march kernel found for the shadow ray, so that a marched shadow ray
 // writes nothing else: bit 31 an SDF hit, bits 29-30 the SDF's sign at the
 // ray's origin + 2 (0: not marched).
-constexpr uint32_t kQueueSlotMask = (1u << 28) - 1u;
+constexpr uint32_t kQueueSlotMask = kMaxPoolSlots - 1u;
 // An entry of the MARCH queues: the slot and, above it, the ray's march group.
 PT_DI uint32_t march_entry(uint32_t slot, uint32_t group) { return slot | (group << 28); }
 static_assert(kMarchGroups <= 16, "march groups must fit the four bits above a slot");

@@ -27,6 +27,10 @@ struct WfPool {
     float4 *s01, *s23, *s49, *s56, *s78, *h01, *m01;  // 2 x 16 B per slot each
 };
 
+// Slots of a pool at most: a queue entry holds its slot in 28 bits, below what
+// the march kernel reports of the ray or the ray's march group (pt_march.cuh).
+constexpr uint32_t kMaxPoolSlots = 1u << 28;
+
 // Entries of a job ring at most (a ring index is stored in 20 bits of the
 // path state).
 constexpr uint32_t kMaxJobRing = 1u << 20;

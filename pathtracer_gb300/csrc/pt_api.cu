@@ -461,7 +461,7 @@ int pt_get_engine(pt_ctx* ctx) { return ctx ? ctx->engine : -1; }
 
 int pt_set_wavefront_pool(pt_ctx* ctx, uint32_t slots) {
     if (!ctx) return PT_ERR_INVALID;
-    if (slots < 1024 || slots > (1u << 28)) return fail(ctx, PT_ERR_INVALID, "pt_set_wavefront_pool: 1024..2^28 slots");
+    if (slots < 1024 || slots > kMaxPoolSlots) return fail(ctx, PT_ERR_INVALID, "pt_set_wavefront_pool: 1024..2^28 slots");
     ctx->pool_cap = slots;
     ctx->staged_knobs = true;
     return PT_OK;
@@ -526,7 +526,7 @@ int pt_get_wavefront_tuning(pt_ctx* ctx, pt_wavefront_tuning* out) {
 
 int pt_set_wavefront_tuning(pt_ctx* ctx, const pt_wavefront_tuning* t) {
     if (!ctx) return PT_ERR_INVALID;
-    if (!t || t->pool_slots < 1024 || t->pool_slots > (1u << 28) || t->march_budget < 1 || t->march_budget > 512 ||
+    if (!t || t->pool_slots < 1024 || t->pool_slots > kMaxPoolSlots || t->march_budget < 1 || t->march_budget > 512 ||
         t->refill_min < 1 || t->refill_min > 32 || t->drain_lanes < 0 || t->drain_lanes > 32 || t->blocks_per_sm < 1 ||
         t->blocks_per_sm > 8 || t->march_inner < 1 || t->march_inner > 16)
         return fail(ctx, PT_ERR_INVALID, "pt_set_wavefront_tuning: a value is out of range");

@@ -362,7 +362,7 @@ int pt_batch_create(pt_batch** out, int device, uint32_t pool_slots, uint32_t ma
     pt_batch* b = new (std::nothrow) pt_batch();
     if (!b) return PT_ERR_OOM;
     b->device = device;
-    b->pool_slots = pool_slots;
+    b->pool_slots = pool_slots < kMaxPoolSlots ? pool_slots : kMaxPoolSlots;
     b->max_passes = max_passes;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
