@@ -303,6 +303,8 @@ void* pt_accum_device_ptr(pt_ctx* ctx);
 
 /* The cudaStream_t the context launches on (as void*), and a way to replace
  * it with a caller-owned stream (NULL restores the context's own stream).
+ * Later calls follow whatever the context has queued on the old stream (a new
+ * stream that is being captured cannot wait for that: the call itself does).
  * A replaced stream must outlive every later call on the context, pt_destroy
  * included (it synchronises the stream): restore NULL before the stream's
  * owner — possibly another context — destroys it. */

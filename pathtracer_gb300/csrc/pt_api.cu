@@ -27,8 +27,7 @@ struct pt_ctx {
     int device = 0;
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
-    cudaEvent_t done = nullptr;
-    cudaEvent_t busy = nullptr;    // after the last dispatch on an engine of the context (pt_set_stream)
+    cudaEvent_t busy = nullptr;    // after the context's last queued work (pt_set_stream)
     KParams* params = nullptr;  // host image of the launch parameters
     bool has_scene = false;
     float* d_cie = nullptr;
@@ -111,11 +110,23 @@ void refresh_plugins(pt_ctx* ctx) {
     ctx->params->s.meta.nplug = ctx->nplug;
 }
 
+// Marks the end of the work queued so far: the context's stream may be replaced
+// before it is done (pt_set_stream).  Not inside a stream capture: other
+// streams cannot wait for an event of one.
+cudaError_t record_busy(pt_ctx* ctx) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(ctx->stream, &capture);
+    if (e != cudaSuccess || capture != cudaStreamCaptureStatusNone) return e;
+    return cudaEventRecord(ctx->busy, ctx->stream);
+}
+
 // Keeps the device copy of the scene (read by the wavefront kernels) in step
 // with the launch-parameter copy (read by the megakernel).
 cudaError_t sync_device_scene(pt_ctx* ctx) {
     if (!ctx->has_scene) return cudaSuccess;
-    return cudaMemcpyAsync(ctx->d_scene, &ctx->params->s, sizeof(KScene), cudaMemcpyHostToDevice, ctx->stream);
+    const cudaError_t e =
+        cudaMemcpyAsync(ctx->d_scene, &ctx->params->s, sizeof(KScene), cudaMemcpyHostToDevice, ctx->stream);
+    return e == cudaSuccess ? record_busy(ctx) : e;
 }
 
 }  // namespace
@@ -128,7 +139,6 @@ constexpr uint64_t kSmallDispatch = 1ull << 18;
 
 static int dispatch_wavefront(pt_ctx* ctx, const pt_push* push);
 static int dispatch_persistent(pt_ctx* ctx, const pt_push* push);
-static cudaError_t record_busy(pt_ctx* ctx);
 static cudaError_t fp64_scratch(pt_ctx* ctx, const pt_push* push, void** scratch, int* sms);
 static int dispatch_jit(pt_ctx* ctx, bool trace);
 static int ensure_jit(pt_ctx* ctx, JitKind kind);
@@ -150,7 +160,6 @@ int pt_create(pt_ctx** out, int device) {
     ctx->device = device;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->done, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->busy, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_cie, sizeof(float) * PT_CIE_TABLE_SIZE);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_rot, sizeof(float) * 9 * PT_MAX_SCENE_OBJECTS);
@@ -197,7 +206,6 @@ int pt_destroy(pt_ctx* ctx) {
     if (ctx->d_fp64) cudaFree(ctx->d_fp64);
     for (auto& cache : ctx->jit)
         for (JitModule& m : cache) pt_jit_unload(m);
-    if (ctx->done) cudaEventDestroy(ctx->done);
     if (ctx->busy) cudaEventDestroy(ctx->busy);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx->params;
@@ -322,6 +330,7 @@ int pt_resize_accum(pt_ctx* ctx, int width, int height) {
     if (ctx->d_accum && width == ctx->width && height == ctx->height) {
         // the same size: zeroed in place, in stream order (no free, no allocation)
         PT_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_accum, 0, bytes, ctx->stream));
+        PT_CUDA_TRY(ctx, record_busy(ctx));
         return PT_OK;
     }
     PT_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
@@ -332,6 +341,7 @@ int pt_resize_accum(pt_ctx* ctx, int width, int height) {
     }
     PT_CUDA_TRY(ctx, cudaMalloc(&ctx->d_accum, bytes));
     PT_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_accum, 0, bytes, ctx->stream));
+    PT_CUDA_TRY(ctx, record_busy(ctx));
     ctx->width = width;
     ctx->height = height;
     return PT_OK;
@@ -410,7 +420,7 @@ int pt_dispatch(pt_ctx* ctx, const pt_push* push) {
     }
     ctx->last_launches = 1;
     PT_CUDA_TRY(ctx, ptk_launch_megakernel(&P, trace, ctx->stream));
-    PT_CUDA_TRY(ctx, cudaEventRecord(ctx->done, ctx->stream));
+    PT_CUDA_TRY(ctx, record_busy(ctx));
     return PT_OK;
 }
 
@@ -444,7 +454,6 @@ int pt_render_fp64(pt_ctx* ctx, const pt_push* push, double* d_sums) {
     }
     P.sums = nullptr;
     PT_CUDA_TRY(ctx, e);
-    PT_CUDA_TRY(ctx, cudaEventRecord(ctx->done, ctx->stream));
     PT_CUDA_TRY(ctx, record_busy(ctx));
     return PT_OK;
 }
@@ -696,8 +705,8 @@ int pt_set_stream(pt_ctx* ctx, void* stream) {
     if (!ctx) return PT_ERR_INVALID;
     const cudaStream_t s = stream ? (cudaStream_t)stream : ctx->own_stream;
     if (s != ctx->stream) {
-        // The scene's device copy, the colour buffer and the engines belong to
-        // the last dispatch that used them until it is done.
+        // The accumulator, the scene's device copy, the colour buffer and the
+        // engines belong to the work queued on the old stream until it is done.
         PT_CUDA_TRY(ctx, cudaSetDevice(ctx->device));
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         PT_CUDA_TRY(ctx, cudaStreamIsCapturing(s, &capture));
@@ -742,15 +751,6 @@ const char* pt_last_error(pt_ctx* ctx) {
 }
 
 }  // extern "C"
-
-// Marks the end of a dispatch that used the context's engines.  Not inside a
-// stream capture: other streams cannot wait for an event of one.
-static cudaError_t record_busy(pt_ctx* ctx) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    const cudaError_t e = cudaStreamIsCapturing(ctx->stream, &capture);
-    if (e != cudaSuccess || capture != cudaStreamCaptureStatusNone) return e;
-    return cudaEventRecord(ctx->busy, ctx->stream);
-}
 
 // The FP64 renderer's scratch; null for a dispatch that takes none, without
 // memory for it, or captured (a graph would keep the pointer).
@@ -827,7 +827,6 @@ static int dispatch_persistent(pt_ctx* ctx, const pt_push* push) {
     PT_CUDA_TRY(ctx, E.resolve(idx));
     ctx->last_iterations = 1;
     ctx->last_launches = E.kernel_launches - launches0;
-    PT_CUDA_TRY(ctx, cudaEventRecord(ctx->done, ctx->stream));
     PT_CUDA_TRY(ctx, record_busy(ctx));
     return PT_OK;
 }
@@ -952,7 +951,6 @@ static int dispatch_wavefront(pt_ctx* ctx, const pt_push* push) {
     for (int e = 0; e < kMax; e++)
         if (*slot[e]) launches1 += (*slot[e])->kernel_launches;
     ctx->last_launches = launches1 - launches0;
-    PT_CUDA_TRY(ctx, cudaEventRecord(ctx->done, ctx->stream));
     PT_CUDA_TRY(ctx, record_busy(ctx));
     return PT_OK;
 }
@@ -1017,6 +1015,6 @@ static int ensure_jit(pt_ctx* ctx, JitKind kind) {
 static int dispatch_jit(pt_ctx* ctx, bool trace) {
     PT_CUDA_TRY(ctx, pt_jit_launch(ctx->jit[kJitMegakernel][(size_t)ctx->jit_cur[kJitMegakernel]], ctx->params, trace,
                                    ctx->stream));
-    PT_CUDA_TRY(ctx, cudaEventRecord(ctx->done, ctx->stream));
+    PT_CUDA_TRY(ctx, record_busy(ctx));
     return PT_OK;
 }
