@@ -133,9 +133,12 @@ struct pt_batch {
     int custom_next = 0;
     JitModule jit;
     bool jit_dirty = false;
-    // March groups (WfJob::group): what the SDF code of each is, the kinds
-    // of built-in plug-ins, or a scene of its own with run-time compiled text.
-    std::vector<uint64_t> groups;
+    // March groups (WfJob::group): the SDF code of each, the kinds of built-in
+    // plug-ins or one scene's run-time compiled text, and its live scenes.
+    struct MarchGroup {
+        uint64_t code = 0;
+        uint32_t scenes = 0;
+    } groups[kMarchGroups];
     uint32_t sdf_kinds = 0;  // plug-in kinds of every scene added (bit k: kind k)
     uint32_t jit_kinds = 0;  // the kinds `jit` was compiled for (PT_SDF_KINDS)
     JitModule jit64;  // the FP64 renderer's megakernel for the same snippets (pt_batch_render_fp64), when needed
@@ -169,6 +172,27 @@ bool count_ok(float v, int max, int* out) {
 BatchPass* pass_at(pt_batch* b, uint32_t j) {
     if (j < b->pass_base || j - b->pass_base >= b->passes.size()) return nullptr;
     return &b->passes[j - b->pass_base];
+}
+
+// The march group of a new scene with SDF code `code`: the live one with that
+// code, else a free one, else the one with the fewest scenes.
+uint32_t take_group(pt_batch* b, uint64_t code) {
+    uint32_t best = 0;
+    for (uint32_t g = 0; g < (uint32_t)kMarchGroups; g++) {
+        if (b->groups[g].scenes > 0 && b->groups[g].code == code) {
+            best = g;
+            break;
+        }
+        if (b->groups[g].scenes < b->groups[best].scenes) best = g;
+    }
+    if (b->groups[best].scenes++ == 0) b->groups[best].code = code;
+    return best;
+}
+
+bool several_groups(const pt_batch* b) {
+    int live = 0;
+    for (const auto& g : b->groups) live += g.scenes > 0;
+    return live > 1;
 }
 
 // The staged engine's march kernel: the batch's run-time compiled one, else
@@ -507,12 +531,6 @@ int add_scene(pt_batch* b, const pt_ubo* ubo, const pt_sdf_plugin* plugins, int 
     S->meta.nplug = nplugins;
     S->meta.custom_base = custom_base;
     pt_derive_cull(S);
-    if (n[5] > 0) {
-        const uint64_t code = custom ? (1ull << 32) + b->scenes.size() : kinds;
-        const size_t g = (size_t)(std::find(b->groups.begin(), b->groups.end(), code) - b->groups.begin());
-        if (g == b->groups.size()) b->groups.push_back(code);
-        bs.group = (uint32_t)(g % kMarchGroups);
-    }
     cudaError_t e = cudaMalloc(&bs.d_scene, sizeof(KScene));
     if (e == cudaSuccess) e = cudaMalloc(&bs.d_cie, sizeof(float) * PT_CIE_TABLE_SIZE);
     if (e == cudaSuccess) e = cudaMemcpyAsync(bs.d_scene, S, sizeof(KScene), cudaMemcpyHostToDevice, b->stream);
@@ -538,6 +556,7 @@ int add_scene(pt_batch* b, const pt_ubo* ubo, const pt_sdf_plugin* plugins, int 
     bs.has_sdf = n[5] > 0;
     bs.custom = custom;
     bs.variant = pt_feature_variant(n);
+    if (bs.has_sdf) bs.group = take_group(b, custom ? (1ull << 32) + b->scenes.size() : kinds);
     // the compiled march kernel holds the code of the kinds seen so far: a
     // scene with another kind needs it compiled again
     b->sdf_kinds |= kinds;
@@ -779,7 +798,7 @@ int pt_batch_step(pt_batch* b, int iterations, int* completed, int capacity, int
         }
     for (int se : {kStaged, kStaged2})
         if (b->engine_live[se])
-            b->engine[se].set_groups((int)std::min(std::max(b->groups.size(), (size_t)1), (size_t)kMarchGroups));
+            b->engine[se].set_groups(several_groups(b) ? kMarchGroups : 1);
     bool busy[kEngines];
     bool any = false;
     for (int e = 0; e < kEngines; e++) {
@@ -1114,6 +1133,7 @@ int pt_batch_release_scene(pt_batch* b, int scene_id) {
     s.d_cie = nullptr;
     s.h_scene.reset();
     s.live = false;
+    if (s.has_sdf) b->groups[s.group].scenes--;
     return PT_OK;
 }
 
