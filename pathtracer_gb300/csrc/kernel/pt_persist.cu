@@ -36,7 +36,7 @@ namespace {
 // instruction fetch more than for anything else (5 to 7 of 13 cycles an
 // issue).  Steps of one class run their code once for full warps.
 constexpr int kPersistSlots = 80;
-constexpr uint32_t kPersistChunk = 256;  // samples a warp claims at once
+constexpr int kPersistChunk = 256;  // samples a warp claims at once, at most
 constexpr int kPersistWarps = kPersistThreads / 32;
 // A path's state, 7 x 16 B a slot (an odd count, so that slots spread over
 // the banks):
@@ -167,7 +167,7 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
     // A staged engine's last paths are spread over every warp: their time is
     // the longest path's, and a warp steps as long as its longest march.
     const int slots = POOL ? warp_slots(share + 1, 1, 1, kPersistSlots) : warp_slots(share, 32, 32, kPersistSlots);
-    const uint32_t chunk = POOL ? min(32u, (uint32_t)share + 1) : share >= 8 * kPersistChunk ? kPersistChunk : (share < 128 ? 32u : (uint32_t)(share / 128 * 32));
+    const uint32_t chunk = POOL ? min(32u, (uint32_t)share + 1) : (uint32_t)warp_chunk(share, kPersistChunk);
     int count[PC_COUNT] = {0, 0, 0, 0};  // warp-uniform: the lists' lengths
     for (int i = lane; i < slots; i += 32) sh.list[warp][PC_END][i] = (uint16_t)(i | (PE_START << 8));
     count[PC_END] = slots;

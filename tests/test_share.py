@@ -11,6 +11,7 @@ from conftest import ROOT
 SHARE_CPP = r"""
 #include "pt_share.h"
 extern "C" int slots(unsigned long long share, int least, int step, int cap) { return warp_slots(share, least, step, cap); }
+extern "C" int chunk(unsigned long long share, int cap) { return warp_chunk(share, cap); }
 """
 
 
@@ -23,6 +24,7 @@ def share(tmp_path_factory):
                     "-I" + os.path.join(ROOT, "pathtracer_gb300", "csrc", "kernel"), "-o", str(lib), str(src)], check=True)
     so = ctypes.CDLL(str(lib))
     so.slots.argtypes = [ctypes.c_uint64] + 3 * [ctypes.c_int]
+    so.chunk.argtypes = [ctypes.c_uint64, ctypes.c_int]
     return so
 
 
@@ -44,3 +46,16 @@ def test_slots_fit_the_arrays(share, source, name, least, step):
         assert s >= n or s == cap, n
         assert s % step == 0 or s == cap, n
         assert s == cap or s < max(n, least) + step, n
+
+
+def test_claims_grow_to_their_limit(share):
+    """Whole warps, never more than the limit, never fewer than for a smaller
+    share, and no more than a quarter of it above the smallest claim."""
+    cap = _constant("pt_persist.cu", "kPersistChunk")
+    last = 0
+    for n in [*range(10001), 2**31 - 1, 2**31, 2**32 - 1, 2**32, 2**63]:
+        c = share.chunk(n, cap)
+        assert 32 <= c <= cap and c % 32 == 0 and c >= last, n
+        assert c == 32 or 4 * c <= n, n
+        last = c
+    assert last == cap
