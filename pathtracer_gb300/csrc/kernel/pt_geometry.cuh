@@ -716,11 +716,10 @@ template <typename V, typename R = SOf<V>> PT_DI R scene_sdf(const KScene& S, V 
 // scene_sdf that also reports the SDF whose material SDFMATERIAL() picks at
 // p (SC:713-719: the last i with !(running minimum < d_i); -1 for none), so
 // a march that converged at p needs only that SDF's material function there.
-// The loop runs over `walk`, a superset of set1 (the union of the sets of
-// lanes that evaluate together), so that lanes whose sets differ evaluate
-// the SDFs they share in the same trip: over each lane's own set, lanes with
-// {0, 1} and lanes with {1} ran SDF 1 in different trips (10.5 of 32 lanes
-// per instruction on menger + terrain).
+// The loop runs over `walk`, a superset of set1 (walk_of), so that lanes whose
+// sets differ evaluate the SDFs they share in the same trip: over each lane's
+// own set, lanes with {0, 1} and lanes with {1} ran SDF 1 in different trips
+// (10.5 of 32 lanes per instruction on menger + terrain).
 // COLD: by calls of the plug-ins' one out-of-line copy (plugin_sdf_cold).
 template <uint32_t KINDS = PT_SDF_KINDS, bool COLD = false, typename V, typename R = SOf<V>>
 PT_DI R scene_sdf_sel(const KScene& S, V p, uint32_t set1, uint32_t walk, int& sel) {
@@ -752,9 +751,16 @@ PT_DI R scene_sdf_sel(const KScene& S, V p, uint32_t set1, uint32_t walk, int& s
     }
     return sdf;
 }
-// The SDFs a lane on its own walks: all of a scene with few, so that lanes
-// of a warp agree; else its set (32 boxes of which a ray meets a few).
-PT_DI uint32_t plugin_walk(const KScene& S, uint32_t set1) { return (S.meta.nplug <= 8) ? plugin_mask(S) : set1; }
+// The SDFs that rays with set1 (not empty) walk: the group of boxes that set1
+// lies in, when all of its SDFs run code of their own, so that lanes whose
+// sets differ agree on the trips; else the lane's own set, whose SDFs lanes
+// evaluate together where their kinds are the same, wherever they stand.  Over
+// all SDFs of the warp's lanes, or of the scene, copies of one SDF take turns.
+// ms so and this way: 16 mengers apart 1280x720x4 staged 14.6, 10.3, 4 of them
+// 160x90 on the plain engine 0.71, 0.50, feature mix (3 kinds apart) 1.23,
+// 1.15; 7 mengers on terrain staged 29.0, 24.4; 3 of them 18.9, 19.4; 8 boxes
+// of two kinds, each meeting the others, 9.0, 10.8.
+PT_DI uint32_t walk_of(const KScene& S, uint32_t set1) { return S.sdf_walk[__ffs(set1) - 1] | set1; }
 // Out-of-line copy for the cold call sites (sign at the origin, normals).
 template <typename V, typename R = SOf<V>>
 static __device__ __noinline__ R scene_sdf_cold(const KScene& S, V p, uint32_t set1) { return scene_sdf(S, p, set1); }
@@ -877,6 +883,7 @@ PT_DI bool sphere_trace(const KScene& S, V3<R> org, V3<R> dir, HitT<R>& h, bool 
         sign.k = k;
         sign.set = set1;
     }
+    uint32_t walk = walk_of(S, set1);
     int hit_sel = -2;  // >= -1 once the march converged (scene_sdf_material_hit)
     // The reference's limits (512 steps, |d| < 1e-4, no distance cap) or the
     // scene's PT_EXT_MARCH ones.
@@ -888,7 +895,7 @@ PT_DI bool sphere_trace(const KScene& S, V3<R> org, V3<R> dir, HitT<R>& h, bool 
     for (int i = 0; i < maxSteps; i++) {
         if (t > tmax) return false;  // past the distance cap: no SDF hit
         int sel;
-        const R radius = scene_sdf_sel(S, p, set1, plugin_walk(S, set1), sel);
+        const R radius = scene_sdf_sel(S, p, set1, walk, sel);
         if (insT > (m_fabs(previousRadius) + m_fabs(radius))) {
             t -= insT;
             omega = PT_LIT(R, 1.0);
@@ -910,6 +917,7 @@ PT_DI bool sphere_trace(const KScene& S, V3<R> org, V3<R> dir, HitT<R>& h, bool 
             t = tMinMax.y + PT_LIT(R, 1e-3);
             tMinMax = v2<R>(R(PT_MAXDIST), R(PT_MAXDIST));
             if (search_sdf(S, fma3s(dir, t, org), invdir, tMinMax, set1)) {
+                walk = walk_of(S, set1);
                 tMinMax.x += t;
                 tMinMax.y += t;
                 t = m_fmax(tMinMax.x, t);

@@ -165,13 +165,14 @@ struct NormalStage {
     float probe[6 * kNormalBatch];
 };
 
-// The SDFs a warp's evaluation walks: the union of its lanes' sets
-// (scene_sdf_sel).  Called by all 32 lanes.
-PT_DI uint32_t warp_walk(bool on, uint32_t set1) {
+// The SDFs a lane's evaluation walks (scene_sdf_sel): its set and, of those
+// that it may walk with others (group: walk_of), the ones in a set of the
+// warp.  Called by all 32 lanes.
+PT_DI uint32_t warp_walk(bool on, uint32_t set1, uint32_t group) {
 #if defined(PT_ONE_SDF)
     return 1u;
 #else
-    return __reduce_or_sync(0xffffffffu, on ? set1 : 0u);
+    return (__reduce_or_sync(0xffffffffu, on ? set1 : 0u) & group) | set1;
 #endif
 }
 
@@ -246,9 +247,9 @@ PT_DI uint32_t take_normals(const PoolView& v, NormalStage& ns, int from, int n,
             a = ns.at[from + r];
             b = ns.of[from + r];
         }
-        const uint32_t walk = warp_walk(on, b.x);
+        const KScene& S = *reinterpret_cast<const KScene*>((uint64_t)b.z | ((uint64_t)b.w << 32));
+        const uint32_t walk = warp_walk(on, b.x, on ? walk_of(S, b.x) : 0u);
         if (on) {
-            const KScene& S = *reinterpret_cast<const KScene*>((uint64_t)b.z | ((uint64_t)b.w << 32));
             const float3 q = probe_point(a, j);
             ns.probe[i] = probe_sdf<KINDS>(S, q, b.x, walk);
         }
@@ -312,7 +313,7 @@ PT_DI void march_rays(const WfArgs& A) {
     float t = 0.0f, insT = 0.0f, omega = 0.0f, prevR = 0.0f, hitdist = 0.0f, k = 0.0f, nplus = 0.0f;
     float3 nv = f3(0.0f, 0.0f, 0.0f);  // nplus, nv: normals on the ray's lane only
     float2 tmm = make_float2(0.0f, 0.0f);
-    uint32_t set1 = 0;
+    uint32_t set1 = 0, group = 0;
     int points = 0, iter = 0;
     bool xmarch = false;  // the ray's scene sets march limits (PT_EXT_MARCH; read from it where used)
     int hit_sel = -2;  // >= -1 once the lane's march converged (scene_sdf_material_hit)
@@ -371,6 +372,7 @@ PT_DI void march_rays(const WfArgs& A) {
                     tmm = make_float2(a1.x, a1.y);
                     k = (float)(int)((saved >> 26) & 3u) - 1.0f;
                     set1 = __float_as_uint(a1.w);
+                    group = walk_of(*Sp, set1);
                     iter = (int)(saved & 1023u);
                     points = (int)((saved >> 10) & 0xffffu);
                     xmarch = (Sp->ext.flags & PT_EXT_MARCH) != 0;
@@ -403,7 +405,7 @@ PT_DI void march_rays(const WfArgs& A) {
             if (!STAGED && phase >= MP_NORMAL0 && phase <= MP_NORMAL5) q = probe_point(p, phase - MP_NORMAL0);
             float val = 0.0f;
             int esel = -1;
-            const uint32_t walk = warp_walk(evalLane, set1);
+            const uint32_t walk = warp_walk(evalLane, set1, group);
             if (evalLane) val = scene_sdf_sel<KINDS>(*Sp, q, set1, walk, esel);
             if (!evalLane) continue;
             if (phase == MP_SIGN) {
@@ -435,6 +437,7 @@ PT_DI void march_rays(const WfArgs& A) {
                         tmm = make_float2(PT_MAXDIST, PT_MAXDIST);
                         const float3 invdir = f3(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
                         if (search_sdf(*Sp, fma3s(dir, t, org), invdir, tmm, set1)) {
+                            group = walk_of(*Sp, set1);
                             tmm.x += t;
                             tmm.y += t;
                             t = fmaxf(tmm.x, t);

@@ -46,7 +46,13 @@ struct KScene {
     // |pos|^2 - r^2 less the margin of the cull test, and a bound on |pos|.
     float4 cull[PT_MAX_SCENE_SPHERES];
     float cull_pmax;
+    // Derived from the SDF boxes and plug-ins on the host (pt_derive_walk): per
+    // SDF slot, the slots that rays near it evaluate in the same trips.
+    uint32_t sdf_walk[PT_MAX_LIVE_SDFS];
 };
+
+// SDFs that a lane on its own walks past at most.
+#define PT_MAX_WALK 8
 
 // The cull test's margin, relative to |org|^2 + |pos|^2 + r^2: 2^-16 = 256
 // float roundings.  The test's own rounding errors and those of the exact
@@ -68,6 +74,42 @@ inline void pt_derive_cull(KScene* S) {
         pmax = std::fmax(pmax, std::sqrt(pp));
     }
     S->cull_pmax = std::nextafter((float)pmax, HUGE_VALF);
+}
+// Fills sdf_walk of a scene whose SDF boxes and plug-ins are set (walk_of).
+inline void pt_derive_walk(KScene* S) {
+    const int n = S->meta.nplug < S->meta.n[5] ? S->meta.nplug : S->meta.n[5];
+    for (int i = 0; i < PT_MAX_LIVE_SDFS; i++) S->sdf_walk[i] = i < n ? 1u << i : 0u;
+    const auto apart = [S](int i, int j) {
+        const float *a = S->sdfs + 6 * i, *b = S->sdfs + 6 * j;
+        for (int k = 0; k < 3; k++)
+            if (2.0f * std::fabs(a[k] - b[k]) > std::fabs(a[3 + k]) + std::fabs(b[3 + k])) return true;
+        return false;
+    };
+    // connected groups of boxes, which a ray's set cannot leave
+    for (int i = 0; i < n; i++)
+        for (int j = 0; j < i; j++) {
+            if (((S->sdf_walk[i] >> j) & 1u) || apart(i, j)) continue;
+            const uint32_t both = S->sdf_walk[i] | S->sdf_walk[j];
+            for (int k = 0; k < n; k++)
+                if ((both >> k) & 1u) S->sdf_walk[k] = both;
+        }
+    // walked together when all of its SDFs run code of their own
+    for (int i = 0; i < n; i++) {
+        const uint32_t group = S->sdf_walk[i];
+        uint32_t kinds = 0;
+        int members = 0;
+        bool copies = false;
+        for (int k = 0; k < n; k++) {
+            if (!((group >> k) & 1u)) continue;
+            const int kind = S->plug[k].kind;
+            members++;
+            copies = copies || (kind != PT_SDF_NONE && kind != PT_SDF_CUSTOM && ((kinds >> kind) & 1u));
+            kinds |= 1u << kind;
+        }
+        if (copies || members > PT_MAX_WALK)
+            for (int k = 0; k < n; k++)
+                if ((group >> k) & 1u) S->sdf_walk[k] = 1u << k;
+    }
 }
 #endif
 

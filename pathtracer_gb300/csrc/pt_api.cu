@@ -108,6 +108,7 @@ void refresh_plugins(pt_ctx* ctx) {
     std::memset(ctx->params->s.plug, 0, sizeof(ctx->params->s.plug));
     std::memcpy(ctx->params->s.plug, ctx->plug, sizeof(pt_sdf_plugin) * (size_t)ctx->nplug);
     ctx->params->s.meta.nplug = ctx->nplug;
+    pt_derive_walk(&ctx->params->s);
 }
 
 // Marks the end of the work queued so far: the context's stream may be replaced

@@ -531,6 +531,7 @@ int add_scene(pt_batch* b, const pt_ubo* ubo, const pt_sdf_plugin* plugins, int 
     S->meta.nplug = nplugins;
     S->meta.custom_base = custom_base;
     pt_derive_cull(S);
+    pt_derive_walk(S);
     cudaError_t e = cudaMalloc(&bs.d_scene, sizeof(KScene));
     if (e == cudaSuccess) e = cudaMalloc(&bs.d_cie, sizeof(float) * PT_CIE_TABLE_SIZE);
     if (e == cudaSuccess) e = cudaMemcpyAsync(bs.d_scene, S, sizeof(KScene), cudaMemcpyHostToDevice, b->stream);

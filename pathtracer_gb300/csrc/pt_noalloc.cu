@@ -113,6 +113,7 @@ int build_scene(const pt_ubo* ubo, const pt_sdf_plugin* plugins, int nplug, KSce
     if (nplug > 0) std::memcpy(S->plug, plugins, sizeof(pt_sdf_plugin) * (size_t)nplug);
     S->meta.nplug = nplug;
     pt_derive_cull(S);
+    pt_derive_walk(S);
     return PT_OK;
 }
 
