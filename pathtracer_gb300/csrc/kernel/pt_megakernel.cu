@@ -1,8 +1,18 @@
 // pt_megakernel.cu — the plain per-pixel spectral path tracer for sm_103a
 // (pt_megakernel_body.cuh): its variants for SDF scenes and traced
-// dispatches, with all math inlined, plus the per-upload rotation setup and
-// the math verification kernel.  The analytic-scene variants live in
-// pt_megakernel_analytic.cu.
+// dispatches, plus the per-upload rotation setup and the math verification
+// kernel.  The analytic-scene variants live in pt_megakernel_analytic.cu.
+//
+// They are bound by instruction fetch, and by how their hot code falls into
+// the instruction cache as much as by its size: with the larger pt_mathf
+// functions called (the plug-ins keep theirs inlined) and the path functions
+// (PT_CALL) inlined, rather than the other way round, the same instructions
+// wait 12 % less.  ms so and this way, plain engine 1024x1024: blob 8 spp
+// 29.0, 26.6, shipped mandelbulb 4 spp 38.0, 37.4, menger + terrain 4 spp 55.2,
+// 53.9, feature mix 4 spp 25.1, 24.8.  Both called, blob 27.6 and menger +
+// terrain 59; with quotients called too, 25.2 and 58.
+#define PTM_OUTLINE
+#define PT_INLINE_PATH
 #include <cuda_runtime.h>
 
 #include "pt_megakernel_body.cuh"

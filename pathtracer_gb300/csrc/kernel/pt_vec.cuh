@@ -34,8 +34,9 @@
 // sphere scene 1024x1024x16 on the megakernel 8.6 -> 7.5 ms, batch of 16
 // sphere jobs 60.2 -> 53.6 ms, Cornell box staged 1.68 -> 1.61 ms.
 // The run-time compiled FP32 kernels hold fewer SDFs and inline them: menger
-// of 4 levels as GLSL on the plain engine 1024x1024x8 37.0 -> 32.8 ms.
-#if defined(PT_JIT_USER_SDF) && !defined(PTG_DOUBLE)
+// of 4 levels as GLSL on the plain engine 1024x1024x8 37.0 -> 32.8 ms.  So do
+// those that define PT_INLINE_PATH (pt_megakernel.cu).
+#if (defined(PT_JIT_USER_SDF) && !defined(PTG_DOUBLE)) || defined(PT_INLINE_PATH)
 #define PT_CALL static __device__ __forceinline__
 #else
 #define PT_CALL static __device__ __noinline__
