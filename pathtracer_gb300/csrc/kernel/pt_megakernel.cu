@@ -126,7 +126,10 @@ cudaError_t ptk_launch_megakernel(const KParams* params, bool trace, cudaStream_
     }
     // The smallest variant that covers the scene's primitive classes.
     const int variant = pt_feature_variant(params->s.meta.n);
-    if (variant != PT_FEAT_ALL) return ptk_launch_megakernel_analytic(params, variant, grid, block, stream);
+    if (variant != PT_FEAT_ALL)
+        return grid.x * grid.y <= (variant ? kSmallFrameBlocks : kSmallSphereBlocks)
+                   ? ptk_launch_megakernel_small(params, variant, grid, block, stream)
+                   : ptk_launch_megakernel_analytic(params, variant, grid, block, stream);
     megakernel<false, PT_FEAT_ALL><<<grid, block, 0, stream>>>(*params);
     return cudaGetLastError();
 }

@@ -31,6 +31,14 @@ uint64_t ptk_fp64_kernels(const pt_push* pc, const void* scratch);  // kernels t
 // translation unit.
 cudaError_t ptk_launch_megakernel_analytic(const KParams* params, int variant, dim3 grid, dim3 block,
                                            cudaStream_t stream);
+cudaError_t ptk_launch_megakernel_small(const KParams* params, int variant, dim3 grid, dim3 block,
+                                        cudaStream_t stream);
+// Blocks up to which they take the small frames' variant: one and a half per
+// SM, or four of spheres and planes alone.  us, small frames' and general
+// variant: full Cornell box 192x108 (168 blocks) 1 spp 122, 136, 16 spp 1660,
+// 1863; 256x144 (288) 138, 139 and 2165, 1935; sphere scene 256x256 (512) 90,
+// 100 and 1124, 1155; 512x288 (1152) 107, 114 and 1464, 1431.
+constexpr unsigned kSmallFrameBlocks = 228, kSmallSphereBlocks = 608;
 
 // Evaluates a pt_mathf function over device arrays (verification hook):
 // fn 0 sin, 1 cos, 2 exp, 3 log, 4 pow(x, y), 5 acos.

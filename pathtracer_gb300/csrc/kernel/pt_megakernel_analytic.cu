@@ -1,9 +1,12 @@
 // pt_megakernel_analytic.cu — the plain megakernel's variants for scenes
 // without SDFs (pt_megakernel_body.cuh).  Their shading calls the larger
 // pt_mathf functions, quotients and roots out of line: these variants are
-// bound by instruction fetch (PT_CALL in pt_vec.cuh).
+// bound by instruction fetch (PT_CALL in pt_vec.cuh).  pt_megakernel_small.cu
+// compiles this file again with quotients and roots inlined.
 #define PTM_OUTLINE
+#if !defined(PT_MK_SMALL)
 #define PT_COMPACT
+#endif
 #include <cuda_runtime.h>
 
 #include "pt_megakernel_body.cuh"
