@@ -242,7 +242,11 @@ int pt_render_fp64(pt_ctx* ctx, const pt_push* push, double* d_sums);
  *     order at the end.  Allocates its scratch on first use.  Dispatches of
  *     scenes without SDFs, and of up to 2^18 samples of built-in SDFs, run on
  *     the persistent kernel instead, unless a staged knob, a trace, stage
- *     times, checks or a drain limit is set.  pt_dispatch may return with work
+ *     times, checks or a drain limit is set.  (A staged knob is any value
+ *     given to pt_set_wavefront_pool, pt_set_wavefront_engines,
+ *     pt_set_march_budget or pt_set_wavefront_tuning, the default too: it
+ *     keeps the context on the staged kernels from then on.  The images are
+ *     the same.)  pt_dispatch may return with work
  *     queued on the stream; pt_set_stream orders the new stream after it.
  *     Refused (PT_ERR_CUDA) in a stream capture: a graph would keep buffers
  *     that later dispatches free or use. */

@@ -1,8 +1,11 @@
-// pt_persist.cu — the persistent path kernel of batches and of dispatches of
-// scenes without SDFs: every warp a wavefront of its own in shared memory.
+// pt_persist.cu — the persistent path kernel, every warp a wavefront of its own
+// in shared memory: batches and dispatches of scenes without SDFs, dispatches of
+// few samples of built-in SDFs, and the last paths of the staged engine
+// (pt_wavefront.cu).
 //
 // pt_persist_checked.cu compiles this file a second time with
-// PT_DEBUG_CHECKS (see pt_wavefront_checked.cu).
+// PT_DEBUG_CHECKS (see pt_wavefront_checked.cu), without the takeover of last
+// paths, which no caller with checks on runs.
 #define PTM_OUTLINE
 #define PT_COMPACT
 #define PT_NO_MARCH_KERNELS
@@ -27,8 +30,8 @@ namespace {
 // that ends writes its colour to its pass's colour buffer, which `resolve`
 // sums in sample order, so results equal the megakernel's bit for bit, and
 // its slot takes the next sample of the launch, across pixels and passes.
-// Suited to scenes without SDFs; SDF marching diverges per lane and belongs
-// to the staged kernels above.
+// A marched ray is marched to its end within a trip, so many samples of SDFs
+// belong to the staged kernels; of few, the longest path decides the time.
 //
 // Why: with a path per lane every trip ran every step (emission, diffuse,
 // mirror and glass surfaces, shadow results, new samples: 60 KB of code) for
@@ -295,8 +298,8 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
                         next = load_staged(A, pool, e, i < nm, i >= nm + np, ps, contrib, q, local, job, r);
                         restored = next >= 0;
                     } else {
-                    job = (s < cjob_end) ? cjob : find_job(A.jobs, A.job_cap, job_lo, job_hi, s);
-                    local = A.jobs[job].local_base + (uint32_t)(s - A.jobs[job].first);
+                        job = (s < cjob_end) ? cjob : find_job(A.jobs, A.job_cap, job_lo, job_hi, s);
+                        local = A.jobs[job].local_base + (uint32_t)(s - A.jobs[job].first);
                     }
                 }
                 cbase += take;
@@ -380,10 +383,7 @@ __global__ void __launch_bounds__(kPersistThreads, FEAT == PT_FEAT_ALL ? 4 : 5)
     persist_paths<FEAT, true, false>(A, &S1);
 }
 
-}  // namespace
-
-namespace {
-
+#if !defined(PT_DEBUG_CHECKS)
 // The last paths of a staged engine, run to their ends here.  Staged, every
 // ray of a path waits for the slowest march of each iteration (64 steps, 25 us
 // of launches): with few paths left an iteration costs the same 60 to 100 us
@@ -406,6 +406,7 @@ __global__ void wf_finish_done(const __grid_constant__ WfArgs A) {
         C.iterations += 1;
     }
 }
+#endif
 
 // Blocks of a persistent kernel that fit on one SM at once, cached.
 template <int FEAT, bool ONE>
@@ -458,7 +459,8 @@ int PTK_WF(ptk_persist_blocks_per_sm)(int variant) {
     }
 }
 
-cudaError_t PTK_WF(ptk_wavefront_finish)(const WfArgs* a, int sms, cudaStream_t stream) {
+#if !defined(PT_DEBUG_CHECKS)
+cudaError_t ptk_wavefront_finish(const WfArgs* a, int sms, cudaStream_t stream) {
     static int blocks = 0;
     if (!blocks) {
         const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(wf_finish),
@@ -475,3 +477,4 @@ cudaError_t PTK_WF(ptk_wavefront_finish)(const WfArgs* a, int sms, cudaStream_t 
     wf_finish_done<<<(a->pool_size + 255) / 256, 256, 0, stream>>>(*a);
     return cudaGetLastError();
 }
+#endif

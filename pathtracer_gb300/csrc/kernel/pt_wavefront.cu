@@ -604,12 +604,16 @@ cudaError_t PTK_WF(ptk_wavefront_launch_resolve)(const WfArgs* a, uint32_t job, 
 cudaError_t PTK_WF(ptk_persist_launch)(const WfArgs* a, int variant, int sms, uint64_t budget,
                                        const KScene* one_scene, cudaStream_t stream);
 int PTK_WF(ptk_persist_blocks_per_sm)(int variant);
-cudaError_t PTK_WF(ptk_wavefront_finish)(const WfArgs* a, int sms, cudaStream_t stream);
 
 extern const WfKernelSet PTK_WF(ptk_wavefront_kernel_set);
 const WfKernelSet PTK_WF(ptk_wavefront_kernel_set) = {
     PTK_WF(ptk_wavefront_launch_init),        PTK_WF(ptk_wavefront_launch_job_add),
     PTK_WF(ptk_wavefront_launch_iteration),   PTK_WF(ptk_wavefront_march),
     PTK_WF(ptk_persist_launch),               PTK_WF(ptk_persist_blocks_per_sm),
-    PTK_WF(ptk_wavefront_launch_resolve),     PTK_WF(ptk_wavefront_finish),
+    PTK_WF(ptk_wavefront_launch_resolve),
+#if !defined(PT_DEBUG_CHECKS)
+    ptk_wavefront_finish,
+#else
+    nullptr,
+#endif
 };

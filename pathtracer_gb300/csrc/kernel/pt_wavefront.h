@@ -177,7 +177,7 @@ struct WfKernelSet {
     cudaError_t (*persist)(const WfArgs*, int, int, uint64_t, const KScene*, cudaStream_t);
     int (*persist_blocks_per_sm)(int);
     cudaError_t (*resolve)(const WfArgs*, uint32_t, const pt_push*, float4*, const float4*, cudaStream_t);
-    cudaError_t (*finish)(const WfArgs*, int, cudaStream_t);
+    cudaError_t (*finish)(const WfArgs*, int, cudaStream_t);  // null in the checked build
 };
 // checked = false: the kernels above; true: the same kernels built with
 // PT_DEBUG_CHECKS (pt_wavefront_checked.cu): every queue, pool-slot, ring and

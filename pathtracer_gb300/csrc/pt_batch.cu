@@ -203,7 +203,7 @@ const void* staged_march_kernel(const pt_batch* b) {
 }
 
 // Creates engine e on first use: a staged engine with the batch's pool,
-// the persistent engine with the smallest pool (it keeps paths in registers).
+// the persistent engine with the smallest pool (it keeps paths in shared memory).
 cudaError_t ensure_engine(pt_batch* b, int e) {
     if (b->engine_live[e]) return cudaSuccess;
     if (!b->estream[e]) {

@@ -196,7 +196,7 @@ struct WfEngine {
     cudaError_t finish();
     // Whether drain() may end with finish() now, given the counters.
     bool can_finish(const WfCounters& c) const {
-        return finish_at > 0 && c.next_sample == c.total && c.live > 0 && c.live <= finish_at &&
+        return finish_at > 0 && kernels->finish && c.next_sample == c.total && c.live > 0 && c.live <= finish_at &&
                c.check_site == PT_CHECK_NONE;
     }
     // Iterations to run before the counters are read again, given what the
