@@ -828,7 +828,7 @@ static int dispatch_persistent(pt_ctx* ctx, const pt_push* push) {
     PT_CUDA_TRY(ctx, E.resolve(idx));
     ctx->last_iterations = 1;
     ctx->last_launches = E.kernel_launches - launches0;
-    PT_CUDA_TRY(ctx, record_busy(ctx));
+    PT_CUDA_TRY(ctx, cudaEventRecord(ctx->busy, ctx->stream));  // not in a capture (pt_dispatch)
     return PT_OK;
 }
 
@@ -952,7 +952,7 @@ static int dispatch_wavefront(pt_ctx* ctx, const pt_push* push) {
     for (int e = 0; e < kMax; e++)
         if (*slot[e]) launches1 += (*slot[e])->kernel_launches;
     ctx->last_launches = launches1 - launches0;
-    PT_CUDA_TRY(ctx, record_busy(ctx));
+    PT_CUDA_TRY(ctx, cudaEventRecord(ctx->busy, ctx->stream));  // not in a capture (pt_dispatch)
     return PT_OK;
 }
 
