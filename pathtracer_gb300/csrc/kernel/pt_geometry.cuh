@@ -758,8 +758,10 @@ PT_DI R scene_sdf_sel(const KScene& S, V p, uint32_t set1, uint32_t walk, int& s
 // all SDFs of the warp's lanes, or of the scene, copies of one SDF take turns.
 // ms so and this way: 16 mengers apart 1280x720x4 staged 14.6, 10.3, 4 of them
 // 160x90 on the plain engine 0.71, 0.50, feature mix (3 kinds apart) 1.23,
-// 1.15; 7 mengers on terrain staged 29.0, 24.4; 3 of them 18.9, 19.4; 8 boxes
-// of two kinds, each meeting the others, 9.0, 10.8.
+// 1.15; 7 mengers on terrain staged 29.0, 24.4; 3 of them 18.9, 19.4; 8 boxes of
+// two kinds, each meeting the others, 9.0, 10.8.  Compiled snippets all run
+// code of their own: 12 in boxes that meet, staged 640x360x4, 2.6 together and
+// 3.3 by own sets, 20 on the plain engine 160x90 0.75 and 1.25.
 PT_DI uint32_t walk_of(const KScene& S, uint32_t set1) { return S.sdf_walk[__ffs(set1) - 1] | set1; }
 // Out-of-line copy for the cold call sites (sign at the origin, normals).
 template <typename V, typename R = SOf<V>>

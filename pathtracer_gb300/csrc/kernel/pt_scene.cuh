@@ -51,9 +51,6 @@ struct KScene {
     uint32_t sdf_walk[PT_MAX_LIVE_SDFS];
 };
 
-// SDFs that a lane on its own walks past at most.
-#define PT_MAX_WALK 8
-
 // The cull test's margin, relative to |org|^2 + |pos|^2 + r^2: 2^-16 = 256
 // float roundings.  The test's own rounding errors and those of the exact
 // test (sphere_hit) add up to less than 100 (intersect_spheres).
@@ -97,16 +94,14 @@ inline void pt_derive_walk(KScene* S) {
     for (int i = 0; i < n; i++) {
         const uint32_t group = S->sdf_walk[i];
         uint32_t kinds = 0;
-        int members = 0;
         bool copies = false;
         for (int k = 0; k < n; k++) {
             if (!((group >> k) & 1u)) continue;
             const int kind = S->plug[k].kind;
-            members++;
             copies = copies || (kind != PT_SDF_NONE && kind != PT_SDF_CUSTOM && ((kinds >> kind) & 1u));
             kinds |= 1u << kind;
         }
-        if (copies || members > PT_MAX_WALK)
+        if (copies)
             for (int k = 0; k < n; k++)
                 if ((group >> k) & 1u) S->sdf_walk[k] = 1u << k;
     }

@@ -75,7 +75,11 @@ inline const char* pt_check_site_name(uint32_t site) {
 // launch (WfEngine::finish_at).  Measured on GB300, ms with 2^14, 2^16 and no
 // such launch: shipped mandelbulb 777x431x16 9.9, 10.3, 11.2; menger + terrain
 // 640x360x4 9.2, 10.0, 11.9; feature mix 641x359x2 (460 K samples) 2.95, 2.65,
-// 3.5: a dispatch of few samples is all tail, and hands over sooner.
+// 3.5: a dispatch of few samples is all tail, and hands over sooner.  With
+// 2^14 and 2^16, up to 2^19 samples: feature mix 640x480x1 3.27, 2.79,
+// 1000x500x1 3.36, 2.94; shipped mandelbulb 4.46, 3.67 and 4.32, 3.88, but
+// 512x400x2 4.92, 5.23; menger + terrain 3.32, 3.30 and 6.68, 7.00; past it
+// (640x480x2) 4.07, 3.80; 4.89, 5.21; 4.03, 4.11.
 constexpr uint32_t kFinishAt = 1u << 14;
 constexpr uint32_t kFinishAtSmall = 1u << 16;
 constexpr uint64_t kFinishSmallTotal = 1ull << 19;

@@ -79,3 +79,26 @@ def test_sets_match_oracle(rt, name):
         images.append(b.read_target(tid))
     for im in images:
         np.testing.assert_array_equal(im[..., :3], images[0][..., :3])
+
+
+def test_many_snippets_equal_on_both_engines(rt):
+    """Ten compiled snippets in boxes that meet, one of them a copy's text: the
+    staged march walks them together; both engines give the same bits."""
+    with open(os.path.join(SCENES, "menger_terrain.json")) as f:
+        d = json.load(f)
+    text = ("float sdf(vec3 p){ vec3 q = abs(p) - vec3(0.%d); return length(max(q, 0.0)) + min(max(q.x, max(q.y, q.z)), 0.0)"
+            " - 0.05; }\nfloat sdfmaterial(vec3 p){ return 2.0; }")
+    d["sdf"] = [{"position": [0.6 * (k % 5 - 2), 1.2, 0.6 * (k // 5)], "boundingSize": [1.6] * 3,
+                 "glsl": text % (30 + min(k, 8))} for k in range(10)]
+    scene = rt["Scene"].parse(json.dumps(d))
+    W, H = 64, 40
+    push = scene.push_constants(W, H, 3, 3, 3, 6)
+    images = []
+    for engine in (0, 1):
+        with rt["Context"](0) as ctx:
+            ctx.set_engine(engine)
+            ctx.bind(scene, rt["cie"])
+            ctx.resize_accum(W, H)
+            ctx.dispatch(push)
+            images.append(ctx.read_accum().view(np.uint32))
+    assert np.array_equal(*images)
