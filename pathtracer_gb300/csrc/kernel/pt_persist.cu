@@ -372,13 +372,20 @@ PT_DI void persist_paths(const WfArgs& A, const KScene* S1) {
     }
 }
 
+// Blocks that fit on an SM: five of the smaller variants, four of those with
+// lenses and cyclides, which spill 148 bytes at five.  ms at five and four,
+// 1920x1080x8: feature mix without SDFs 9.69, 8.51, its lenses alone 4.82, 4.63,
+// twelve cyclides 10.5, 9.8; 800x600x1 0.43, 0.38, 0.24, 0.21, 0.68, 0.61.
 template <int FEAT>
-__global__ void __launch_bounds__(kPersistThreads, FEAT == PT_FEAT_ALL ? 4 : 5) wf_persist(const __grid_constant__ WfArgs A) {
+constexpr int kPersistBlocks = (FEAT & PT_FEAT_LENS) || (FEAT & PT_FEAT_SDF) ? 4 : 5;
+
+template <int FEAT>
+__global__ void __launch_bounds__(kPersistThreads, kPersistBlocks<FEAT>) wf_persist(const __grid_constant__ WfArgs A) {
     persist_paths<FEAT, false, false>(A, nullptr);
 }
 
 template <int FEAT>
-__global__ void __launch_bounds__(kPersistThreads, FEAT == PT_FEAT_ALL ? 4 : 5)
+__global__ void __launch_bounds__(kPersistThreads, kPersistBlocks<FEAT>)
     wf_persist_one(const __grid_constant__ WfArgs A, const __grid_constant__ KScene S1) {
     persist_paths<FEAT, true, false>(A, &S1);
 }
