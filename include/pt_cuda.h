@@ -240,7 +240,8 @@ int pt_render_fp64(pt_ctx* ctx, const pt_push* push, double* d_sums);
  *     path slots in device memory; compacted ray queues per stage and a
  *     persistent SDF-march kernel; per-sample XYZ summed per pixel in sample
  *     order at the end.  Allocates its scratch on first use.  Dispatches of
- *     scenes without SDFs, and of up to 2^18 samples of built-in SDFs, run on
+ *     scenes without SDFs (with cyclides beside boxes or lenses: of up to
+ *     3 * 2^19 samples), and of up to 2^18 samples of built-in SDFs, run on
  *     the persistent kernel instead, unless a staged knob, a trace, stage
  *     times, checks or a drain limit is set.  (A staged knob is any value
  *     given to pt_set_wavefront_pool, pt_set_wavefront_engines,

@@ -138,6 +138,17 @@ cudaError_t sync_device_scene(pt_ctx* ctx) {
 // 8.2 and 6.8; menger + terrain 160x90x1 1.61 and 3.27, 320x180x2 2.91 and 3.87.
 constexpr uint64_t kSmallDispatch = 1ull << 18;
 
+// Samples up to which a dispatch of a scene without SDFs that mixes cyclides
+// with boxes or lenses takes it: the steps of such a scene run more code than
+// the instruction cache holds, which the staged kernels run a stage at a time.
+// ms, persistent and staged, 800x600 at 2, 4, 6 spp, 1920x1080x8: feature mix
+// without SDFs 0.67 and 0.93, 1.30 and 1.33, 1.91 and 1.73, 8.5 and 7.5; three
+// times its objects 1.09 and 1.28, 2.07 and 1.96, 2.98 and 2.59, 13.5 and 12.2;
+// without boxes 0.56 and 0.84, 1.04 and 1.15, 1.51 and 1.50, 6.7 and 6.3.
+// Without cyclides 0.46 and 0.80, 0.87 and 1.12, 1.27 and 1.41, 5.7 and 5.9:
+// every other scene without SDFs stays in the persistent kernel.
+constexpr uint64_t kMixedDispatch = 3ull << 19;
+
 static int dispatch_wavefront(pt_ctx* ctx, const pt_push* push);
 static int dispatch_persistent(pt_ctx* ctx, const pt_push* push);
 static cudaError_t fp64_scratch(pt_ctx* ctx, const pt_push* push, void** scratch, int* sms);
@@ -406,7 +417,8 @@ int pt_dispatch(pt_ctx* ctx, const pt_push* push) {
     }
     if (wavefront) {
         // A scene without SDFs has nothing for the staged kernels to sort:
-        // its paths stay on chip in the persistent kernel (dispatch_persistent).
+        // its paths stay on chip in the persistent kernel (dispatch_persistent),
+        // but for many of a scene that mixes primitives (kMixedDispatch).
         // Whatever asks for the staged kernels themselves gets them: traces,
         // stage times, index checks, a drain limit or a staged knob.
         const bool plain_call = !trace && !ctx->stage_timing && !ctx->device_checks && ctx->drain_limit == 0;
@@ -415,7 +427,10 @@ int pt_dispatch(pt_ctx* ctx, const pt_push* push) {
         // slowest march of each step (measured: kSmallDispatch).
         const uint64_t total = (uint64_t)push->resolution[0] * (uint64_t)push->resolution[1] *
                                (uint64_t)push->samplesPerFrame;
-        const bool on_chip = P.s.meta.n[5] == 0 || (ctx->custom.empty() && total <= kSmallDispatch);
+        const int* n = P.s.meta.n;
+        const bool mixed = n[4] > 0 && (n[2] > 0 || n[3] > 0);
+        const bool on_chip = n[5] == 0 ? (!mixed || total <= kMixedDispatch)
+                                       : (ctx->custom.empty() && total <= kSmallDispatch);
         if (on_chip && plain_call && !ctx->staged_knobs) return dispatch_persistent(ctx, push);
         return dispatch_wavefront(ctx, push);
     }
