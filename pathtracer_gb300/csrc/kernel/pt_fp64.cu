@@ -26,10 +26,11 @@ namespace {
 // intersects the rays they go on with together.  A sample's colour goes to
 // scratch; fp64_sum adds a pixel's in sample order, as the megakernel does.
 // The megakernel also left SMs empty: 128x128 pixels are 128 blocks of 152
-// SMs, 64x64 32.  ms, megakernel and this: full Cornell box 128x128x4 5.10,
-// 2.74, 64x64x1 1.23, 1.20,
-// 512x512x16 221, 109; menger + terrain 128x128x4 86.7, 31.6; shipped
-// mandelbulb 256x256x16 606, 196.
+// SMs, 64x64 32.  ms of a call by itself, an image's first samples, megakernel
+// and this: full Cornell box 128x128x4 5.08, 2.83, 64x64x1 1.23, 1.19,
+// 512x512x16 221, 109; menger + terrain 128x128x4 86.6, 27.6; shipped mandelbulb
+// 128x128x4 68.5, 36.8, 256x256x16 606, 196.  (Another
+// frame's samples of the first, perf/cases.py's: 4.17, 2.26.)
 constexpr int kFp64Slots = 64;
 constexpr int kFp64Threads = 128, kFp64Warps = kFp64Threads / 32;
 constexpr int kFp64Refill = 16;     // ended paths gathered before new samples start together

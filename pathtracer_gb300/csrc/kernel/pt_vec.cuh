@@ -31,8 +31,9 @@
 // and at 0.3 to 0.5 beyond (measured on GB300 with unrolled loops of 4 to
 // 192 KB), and the smallest of them held 99 KB.  With emission, the CIE fit
 // and table, glass and the two lens faces in one copy each it holds 77 KB:
-// sphere scene 1024x1024x16 on the megakernel 8.6 -> 7.5 ms, batch of 16
-// sphere jobs 60.2 -> 53.6 ms, Cornell box staged 1.68 -> 1.61 ms.
+// sphere scene 1024x1024x16 on the megakernel 8.2 -> 7.5 ms, batch of 16
+// sphere jobs 55.9 -> 53.6 ms, Cornell box staged 1.66 -> 1.61 ms, the sphere
+// loop's first pass (intersect_spheres) among the change.
 // The run-time compiled FP32 kernels hold fewer SDFs and inline them: menger
 // of 4 levels as GLSL on the plain engine 1024x1024x8 37.0 -> 32.8 ms.  So do
 // those that define PT_INLINE_PATH (pt_megakernel.cu).
